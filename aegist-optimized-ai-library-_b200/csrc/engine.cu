@@ -107,6 +107,9 @@ static size_t dtype_size(const std::string& d) {
     return 0;
 }
 
+// places for `picks` sorted picks of up to `experts` experts, every expert's list starting at a multiple of UQ_G; bytes of their planes
+static size_t q4_slots(int picks, int experts) { return ((size_t)picks + (size_t)(UQ_G - 1) * std::min(experts, picks) + UQ_G - 1) / UQ_G * UQ_G; }
+static size_t q4_plane_bytes(size_t slots, int K) { return (size_t)((K + UQ_KB - 1) / UQ_KB) * (slots / UQ_G) * UQ_GBYTES; }
 constexpr int g_tc_warps = 16;   // compute warps per block of k_tcgemv
 static int down_row_blocks(int D) { return (D + DOWN_ROWS - 1) / DOWN_ROWS; }
 
@@ -171,7 +174,7 @@ struct b2_engine {
     int *g_list = nullptr, *g_slot = nullptr, *g_chunk = nullptr;
     __half* acth = nullptr;
     float *xsum_tok = nullptr, *xsum_act = nullptr;
-    int8_t* sq = nullptr; float *sq_scale = nullptr, *sq_sum = nullptr;   // planes of the sorted picks (k_umma_q4)
+    uint8_t* sq = nullptr; float *sq_scale = nullptr, *sq_sum = nullptr;   // planes of the sorted picks (k_umma_q4)
     int cap_small = 0, cap_big = 0;
     const uint8_t** top_ptr = nullptr;       // [B][TOPK] expert blobs of the current layer's picks (k_moe_gu1 -> k_moe_down1)
     int8_t* actq = nullptr;                  // [B * TOPK][4][I] digit planes of act
@@ -232,7 +235,7 @@ struct b2_engine {
         int8_t* uq_i = nullptr; uint16_t* uq_b = nullptr; float* uq_scale = nullptr; int uq_passes = 0;
         int *g_list = nullptr, *g_slot = nullptr, *g_chunk = nullptr;
         float *xsum_tok = nullptr, *xsum_act = nullptr;
-        int8_t* sq = nullptr; float *sq_scale = nullptr, *sq_sum = nullptr;
+        uint8_t* sq = nullptr; float *sq_scale = nullptr, *sq_sum = nullptr;
         int cap_small = 0, cap_big = 0, nsplit = 1, attn_tiles = 1;
         int* csel = nullptr; float *cselw = nullptr, *cscore = nullptr, *core_y = nullptr;
     } pc;
@@ -575,13 +578,14 @@ int b2_engine::finish() {
         const size_t P = Bg * c.TOPK;
         cap_small = (int)std::min<size_t>(P, c.E / ep_world);
         cap_big = (int)(P / (GQ_SMALL + 1)) + 1;
-        CU(dalloc(&g_list, P)); CU(dalloc(&g_slot, P));
+        CU(dalloc(&g_list, q4_slots((int)P, c.E / ep_world))); CU(dalloc(&g_slot, P));
         CU(dalloc(&g_chunk, (size_t)3 * (cap_small + cap_big) + 2));
         CU(dalloc((uint16_t**)&acth, P * 2 * c.I));
         CU(dalloc(&xsum_tok, Bg * (c.D / 64)));
         CU(dalloc(&xsum_act, P * std::max(1, c.I / 64)));
-        CU(dalloc(&sq, (size_t)UM_PI * P * std::max(c.D, c.I)));
-        CU(dalloc(&sq_scale, P)); CU(dalloc(&sq_sum, P * (size_t)(std::max(c.D, c.I) / 64 + 1)));
+        const size_t slots = q4_slots((int)P, c.E / ep_world);
+        CU(dalloc(&sq, q4_plane_bytes(slots, std::max(c.D, c.I))));
+        CU(dalloc(&sq_scale, slots)); CU(dalloc(&sq_sum, slots * (size_t)(std::max(c.D, c.I) / 64 + 1)));
     }
     CU(dalloc(&ypart, Bg * (c.TOPK + 1) * c.D));
     CU(dalloc(&d_dcounter, Bg * down_row_blocks(c.D)));
@@ -979,7 +983,7 @@ struct ExpertMmaCtx {
     int* list; int* slot; int* chunk; int cap_small, cap_big;
     __half* xh; __half* acth; float* xsum_tok; float* xsum_act;
     // the tcgen05 kernel's operands: planes of the sorted picks, and where this GPU's expert blobs lie
-    int8_t* sq; float* sq_scale; float* sq_sum; int slots;
+    uint8_t* sq; float* sq_scale; float* sq_sum; int slots;
     const uint8_t* experts; size_t expert_bytes; int per, e0;
 };
 static void chunk_tables(const ExpertMmaCtx& m, ChunkTable& small, ChunkTable& big) {
@@ -1006,7 +1010,7 @@ static cudaError_t launch_q4(Q4Args q, const ChunkTable& small, const ChunkTable
 // The shapes k_umma_q4 takes, and the tensor maps of its two launches (gate/up pairs, down): the pick lists are cut for the kernel
 // that reads them, so whether it can run is known before they are.
 static bool umma_q4_maps(const ExpertArgs& a, const ExpertMmaCtx& m, int P, UmmaQ4Args (&u)[2]) {
-    if (!m.sq || !m.experts || P > m.slots || m.expert_bytes % 16 != 0 || a.I > 512) return false;       // k_prep_q_slots<2>: 512 values
+    if (!m.sq || !m.experts || q4_slots(P, m.per) > m.slots || m.expert_bytes % 16 != 0 || a.I > 512) return false;       // k_prep_q_slots<2>: 512 values
     for (int i = 0; i < 2; i++) {
         const bool pair = i == 0;
         const int K = pair ? a.D : a.I, row_blocks = pair ? a.I : a.D / 2;
@@ -1015,9 +1019,9 @@ static bool umma_q4_maps(const ExpertArgs& a, const ExpertMmaCtx& m, int P, Umma
         if (K % UQ_KB != 0 || K > 64 * UQ_MAXG || row_blocks % UM_M != 0 || ((uintptr_t)base & 15) || (u[i].off_s | u[i].off_m) % 8 != 0) return false;
         const cuuint64_t dims[3] = {(cuuint64_t)K / 2, (cuuint64_t)(pair ? 2 * a.I : a.D), (cuuint64_t)m.per};
         const cuuint64_t strides[2] = {(cuuint64_t)K / 2, (cuuint64_t)m.expert_bytes};
-        const cuuint32_t box[3] = {UQ_KB / 2, 64, 1};
-        if (!encode_byte_map(&u[i].wmap, 3, base, dims, strides, box) ||
-            !byte_matrix_map(&u[i].xmap, m.sq, (uint64_t)(K / UM_BK) * m.slots * UM_PI, UM_BK, UQ_BOX)) return false;
+        const cuuint32_t box[3] = {UQ_KB / 2, UM_M, 1};
+        if (!encode_byte_map(&u[i].wmap, 3, base, dims, strides, box)) return false;
+        u[i].wide = (K / 64) % 8 == 0 && (u[i].off_s | u[i].off_m) % 16 == 0;
     }
     return true;
 }
@@ -1025,16 +1029,15 @@ static bool umma_q4_maps(const ExpertArgs& a, const ExpertMmaCtx& m, int P, Umma
 static cudaError_t launch_umma_q4(const ExpertArgs& a, const ExpertMmaCtx& m, const GroupArgs& g, bool pair, int P, UmmaQ4Args& u, int nsm, cudaStream_t st) {
     cudaError_t e;
     const int K = pair ? a.D : a.I, rows = pair ? a.I : a.D;
-    float* const xsum = m.sq_sum;                            // [slots][K / 64]
     PrepSlotsArgs p{};
     p.src = pair ? a.x : a.act; p.stride = pair ? a.x_stride : a.I; p.by_pick = pair ? 0 : 1; p.topk = a.topk;
-    p.norm_w = pair ? a.norm_w : nullptr; p.eps = a.eps; p.K = K; p.rows = pair ? P / a.topk : P; p.slot = g.slot; p.qi = m.sq; p.slots = m.slots;
-    p.xscale = m.sq_scale; p.xsum = xsum;
+    p.norm_w = pair ? a.norm_w : nullptr; p.eps = a.eps; p.K = K; p.rows = pair ? P / a.topk : P; p.slot = g.slot; p.planes = m.sq; p.slots = m.slots;
+    p.xscale = m.sq_scale; p.xsum = m.sq_sum;
     e = pair ? launch_k(k_prep_q_slots<8>, dim3(p.rows), dim3(256), 0, st, p) : launch_k(k_prep_q_slots<2>, dim3((P + 3) / 4), dim3(256), 0, st, p);
     if (e != cudaSuccess) return e;
     u.eptr = a.eptr; u.list = g.list; u.small = g.small; u.big = g.big; u.topk = a.topk; u.pair = pair ? 1 : 0; u.rows = rows; u.K = K;
     u.up_row0 = a.I; u.e0 = m.e0;
-    u.slots = m.slots; u.xscale = m.sq_scale; u.xsum = xsum; u.out = pair ? a.act : a.ypart; u.err = a.err;
+    u.slots = m.slots; u.planes = m.sq; u.xscale = m.sq_scale; u.xsum = m.sq_sum; u.out = pair ? a.act : a.ypart; u.err = a.err;
     if ((e = opt_in_smem(k_umma_q4, UQ_SMEM)) != cudaSuccess) return e;
     g_umma_launches++;
     return launch_k(k_umma_q4, dim3(nsm), dim3(UQ_THREADS), UQ_SMEM, st, u);
@@ -1051,6 +1054,7 @@ static cudaError_t launch_experts_mma(const ExpertArgs& a, int T, const ExpertMm
     const bool q4_umma = umma_q4_maps(a, m, P, u);            // else (K not a multiple of 256, no tensor maps): k_mma_q4
     g.small_n = q4_umma ? UQ_SMALL : GQ_SMALL;
     g.big_n = q4_umma ? UQ_TT : GQ_BIG;
+    g.align = q4_umma ? UQ_G : 1;
     if ((e = launch_k(k_group_picks, dim3(1), dim3(1024), 0, st, g)) != cudaSuccess) return e;
     if (q4_umma) {
         if ((e = launch_umma_q4(a, m, g, true, P, u[0], nsm, st)) != cudaSuccess) return e;
@@ -1371,7 +1375,7 @@ int b2_engine::enqueue_step(cudaStream_t st, bool count, int chunk_T, bool chunk
             const int Tg = B * ep_world;
             const bool grouped = xh && Tg >= BATCH_GEMM_MIN && grouped_shape_ok(c, Tg);
             const ExpertMmaCtx mctx{g_list, g_slot, g_chunk, cap_small, cap_big, xh, acth, xsum_tok, xsum_act,
-                                    chunk ? pc.sq : sq, chunk ? pc.sq_scale : sq_scale, chunk ? pc.sq_sum : sq_sum, Tg * c.TOPK,
+                                    chunk ? pc.sq : sq, chunk ? pc.sq_scale : sq_scale, chunk ? pc.sq_sum : sq_sum, (int)q4_slots(Tg * c.TOPK, c.E / ep_world),
                                     l.experts, c.expert_bytes(), c.E / ep_world, ep_rank * (c.E / ep_world)};
             if (ep_world == 1) {
                 x2.x = x; x2.x_stride = c.D; x2.top_idx = a.top_idx; x2.top_w = a.top_w; x2.idx_stride = c.TOPK;
@@ -1501,12 +1505,13 @@ int b2_engine::ensure_chunk_bufs(int T) {
     want(&pc.uq_scale, (size_t)pc.uq_passes * UM_TOK);
     pc.cap_small = (int)std::min<size_t>(P, c.E);
     pc.cap_big = (int)(P / (GQ_SMALL + 1)) + 1;
-    want(&pc.g_list, P); want(&pc.g_slot, P);
+    want(&pc.g_list, q4_slots((int)P, c.E)); want(&pc.g_slot, P);
     want(&pc.g_chunk, (size_t)3 * (pc.cap_small + pc.cap_big) + 2);
     want((uint16_t**)&pc.acth, P * 2 * c.I);
     want(&pc.xsum_tok, (size_t)W * (c.D / 64));
     want(&pc.xsum_act, P * std::max(1, c.I / 64));
-    want(&pc.sq, (size_t)UM_PI * P * std::max(c.D, c.I)); want(&pc.sq_scale, P); want(&pc.sq_sum, P * (size_t)(std::max(c.D, c.I) / 64 + 1));
+    const size_t slots = q4_slots((int)P, c.E);
+    want(&pc.sq, q4_plane_bytes(slots, std::max(c.D, c.I))); want(&pc.sq_scale, slots); want(&pc.sq_sum, slots * (size_t)(std::max(c.D, c.I) / 64 + 1));
     want(&pc.csel, (size_t)W * c.cores_active); want(&pc.cselw, (size_t)W * c.cores_active);
     want(&pc.cscore, (size_t)W * (c.n1 + c.n2)); want(&pc.core_y, (size_t)W * c.D);
     size_t total = 0;

@@ -387,33 +387,56 @@ __device__ __forceinline__ void router_topk_warp(const float* __restrict__ logit
 
 // ---- bulk asynchronous copies (TMA) into a shared-memory ring, tracked by mbarriers ----
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// Barriers go by pointer or by their shared-memory address: turning a pointer into an address reads a special register (some 30 clocks), and
+// the compiler does it again at every use, so a kernel whose roles hand over often keeps one address in a register (held).
+__device__ __forceinline__ uint32_t smem_u32(uint32_t a) { return a; }
+__device__ __forceinline__ uint32_t held(uint32_t x) { asm volatile("" : "+r"(x)); return x; }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
+template <typename B>
+__device__ __forceinline__ void mbar_expect_tx(B bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+template <typename B>
+__device__ __forceinline__ void mbar_arrive(B bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// the same by the threads that say so: one predicated instruction, no branch and no reconvergence behind it
+template <typename B>
+__device__ __forceinline__ void mbar_arrive_if(bool yes, B bar) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(smem_u32(bar)), "r"((uint32_t)yes) : "memory");
+}
+template <typename B>
+__device__ __forceinline__ bool mbar_try(B bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
 }
 // Wait for a phase of an mbarrier of this block. The wait is bounded: if the phase has not completed
 // after a very long time (a copy that never lands), *err is set and the caller goes on with whatever
 // the buffer holds, so that the kernel always terminates.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err, int limit = 1 << 22) {
-    for (int spin = 0; spin < limit; spin++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
+// The first two tries stand outside the loop: a try blocks for some 5 us when a whole warp makes it, and a warp that is past a loop
+// wakes up 320 clocks after the last arrival, one that is past a plain branch 114 (a phase that is already over: 130 and 55). A wait
+// by one thread of a warp never blocks and polls every 170 clocks, so whole warps wait where it matters. `limit` tries, and about a
+// quarter of a second: a blocking try makes many of them last longer than that.
+template <typename B>
+__device__ __forceinline__ bool mbar_wait(B bar, uint32_t parity, int* err, int limit = 1 << 22) {
+    if (mbar_try(bar, parity)) return true;
+    if (mbar_try(bar, parity)) return true;
+    const long long t0 = clock64();
+    for (int spin = 2; spin < limit && clock64() - t0 < (1ll << 29); spin++)
+        if (mbar_try(bar, parity)) return true;
     if (err) atomicExch(err, 3);
     return false;
 }
 // One contiguous copy global -> shared; src, dst 16-byte aligned, bytes a multiple of 16.
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+template <typename D, typename B>
+__device__ __forceinline__ void bulk_load(D dst, const void* src, uint32_t bytes, B bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
                  "l"(src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");

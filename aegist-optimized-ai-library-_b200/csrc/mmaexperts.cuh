@@ -38,10 +38,11 @@ struct GroupArgs {
     const int* top_idx;           // [T][idx_stride]
     int idx_stride, T, topk, E;
     const uint8_t* const* eptr;   // only experts resident here are grouped
-    int* list;                    // [P] pick ids (t * topk + r) sorted by expert, pick order inside an expert
+    int* list;                    // pick ids (t * topk + r) sorted by expert, pick order inside an expert
     int* slot;                    // [P] a pick's position in the list, or -1 (its expert is not resident here)
     ChunkTable small, big;
     int small_n, big_n;           // most picks of a small and of a big chunk
+    int align;                    // an expert's list starts at a multiple of this
 };
 
 // one block of 1024 threads. An expert's list is in pick order: which chunk a pick falls into decides the order in which
@@ -67,13 +68,14 @@ __global__ void __launch_bounds__(1024) k_group_picks(const GroupArgs a) {
     __syncthreads();
     // per expert: big chunks of up to big_n picks while more than small_n are left, then one small chunk of the rest;
     // exclusive prefix sums over the experts of the pick counts and of the two chunk counts (256 threads)
-    int cnt = 0, nb = 0, ns = 0, x0 = 0, x1 = 0, x2 = 0;
+    int cnt = 0, room = 0, nb = 0, ns = 0, x0 = 0, x1 = 0, x2 = 0;
     if (threadIdx.x < 256) {
         const int e = threadIdx.x;
         cnt = e < a.E ? s_cnt[e] : 0;
         nb = cnt > a.small_n ? (cnt - a.small_n + a.big_n - 1) / a.big_n : 0;
         ns = (cnt - nb * a.big_n) > 0 ? 1 : 0;
-        x0 = cnt; x1 = nb; x2 = ns;
+        room = (cnt + a.align - 1) / a.align * a.align;
+        x0 = room; x1 = nb; x2 = ns;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int y0 = __shfl_up_sync(0xffffffffu, x0, o), y1 = __shfl_up_sync(0xffffffffu, x1, o), y2 = __shfl_up_sync(0xffffffffu, x2, o);
@@ -86,7 +88,7 @@ __global__ void __launch_bounds__(1024) k_group_picks(const GroupArgs a) {
         const int e = threadIdx.x;
         int b0 = 0, b1 = 0, b2 = 0;
         for (int w = 0; w < warp; w++) { b0 += s_w[0][w]; b1 += s_w[1][w]; b2 += s_w[2][w]; }
-        const int off = b0 + x0 - cnt, cb0 = b1 + x1 - nb, cs0 = b2 + x2 - ns;
+        const int off = b0 + x0 - room, cb0 = b1 + x1 - nb, cs0 = b2 + x2 - ns;
         s_off[e] = off;
         int s0 = 0, left = cnt;
         for (int k = 0; k < nb; k++) {

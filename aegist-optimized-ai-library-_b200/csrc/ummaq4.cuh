@@ -1,42 +1,42 @@
 // k_umma_q4: the 4-bit experts of a step (6 or more tokens) or prompt chunk as a grouped Blackwell tensor-core GEMM
 // (the reference's expert GEMMs for more than 8 tokens, aegist_rs/kernels/hybrid.cu:461-549).
 //
-// k_group_picks has sorted the step's picks by expert and cut every expert's list into chunks of at most 20 picks. A
-// unit of work is (chunk, two blocks of 128 weight rows): out[pick][row] = sum_k w[row][k] x[pick][k] for the chunk's
-// picks, with w = code * scale_g + min_g per 64-value group g (aegist/hybrid.py ExpertBank), so
+// k_group_picks has sorted the step's picks by expert, every expert's list starting at a multiple of eight, and cut the lists into
+// chunks of at most 32 picks. A unit of work is (chunk, two blocks of 128 weight rows): out[pick][row] = sum_k w[row][k] x[pick][k]
+// for the chunk's picks, with w = code * scale_g + min_g per 64-value group g (aegist/hybrid.py ExpertBank), so
 //     sum_k w x = sum_g ( scale_g * sum_{k in g} code x  +  min_g * sum_{k in g} x ).
-// The integer sums of a group must not mix with another group's, so every group gets its own accumulator columns in
-// tensor memory and the epilogue folds them with the group's fp16 scale. The two row blocks are a unit's gate and up
-// rows (or two neighbouring blocks of down rows), and the K loop is outside them:
+// The sums of a group must not mix with another group's, so every group gets its own accumulator columns in tensor memory and the
+// epilogue folds them with the group's fp16 scale. The two row blocks are a unit's gate and up rows (or two neighbouring blocks of
+// down rows), and the K loop is outside them.
 //
-//   producer warp     TMA tensor copies per K step (256 codes = 4 groups): once the three int8 digit planes of the chunk's
-//                     picks (4 KB per 32 plane rows and 128 values, consecutive memory: the planes are stored in sorted-pick
-//                     order), then per row block the packed codes of 128 rows (128 bytes each, through a 3-D tensor map
-//                     [expert][row][byte], 128-byte swizzle). Two rings: 5 x 16 KB of codes, 4 x 16 KB of planes
-//   2 table warps     the picks' scales, group sums and output rows of the next unit, and per K step the scale and min of the
-//                     256 rows' four groups, 8 bytes each, into a third ring, one row next to the other
-//   4 converter warps thread = weight row = TMEM lane: the codes' nibbles -> int8 (0..15) straight into tensor memory
-//                     (tcgen05.st, one of four buffers of 64 columns), where tcgen05.mma takes its A operand from; the ring
-//                     slot is free as soon as the codes are in registers
-//   MMA warp          per group two tcgen05.mma (kind::i8, M 128, N 32 or 64, K 32) into that group's columns of one of two
-//                     accumulator buffers of 128 columns: the four groups of a chunk of up to 10 picks, two of a larger one
-//   16 epilogue warps thread = weight row = TMEM lane, four warps to a lane quarter, each with a share of the picks: of a
-//                     small chunk two warps to a row block (an accumulator buffer each), of a larger one five picks of both
-//                     row blocks: tcgen05.ld of two groups, planes combined per pick, times the row's group scale, plus
-//                     the group minimum times the pick's group sum, group after group. A pick's sum has this one order in chunks of
-//                     every size (with the groups split over warps it had another, which k_delta_prompt's note on orders
-//                     applies to). After the last K step the sums meet in shared memory; then activation scale and
-//                     silu(gate) * up, or the picks' output rows
+// Arithmetic. An activation is s q / 2^14 with q a whole number below 2^21 in magnitude (22 bits of the pick's largest value), and q is
+// two whole numbers of 11 bits, q = 2048 h + l, which fp16 holds exactly. A code (0..15) is an fp16 as it lies in its nibble: the bits
+// 0x000c are the subnormal c 2^-24 and 0x00c0 is c 2^-20, so two masks and a shift turn a nibble pair into operands; the planes of
+// the values that meet the second kind carry 2^-4. Products and the sums of 64 of them are below 2^20 units: exact in the tensor
+// core's fp32 accumulators, whatever its order. One fma joins the planes (rounding once, as a conversion of the whole number would).
+// With int8 planes (three digits, half as many products) the epilogue was what bound the kernel: three columns instead of two per
+// pick, two integer products and a conversion instead of half an fma: 2700 clocks per row block and K step of 20 picks.
 //
-// What bounds it, per row block and K step (16 KB of codes, 2 KB of scales): 0.42 us of HBM at the SM's share, or, with full
-// chunks, the hand-over of buffers: the products of a row block and K step wait for their codes to be unpacked behind the
-// products that used the code buffer before (about 1000 clocks of converter work, commit and wake-up), and an accumulator
-// buffer takes about 1100 clocks until it may be written again. Tensor memory holds four code buffers and two accumulators;
-// two and three took 1.238 against 1.217 ms per 4-layer step at 64 sequences and 1.127 against 1.066 for a 45-token prompt.
-// Eight converter warps were no faster (the chain is latency, not issue). Hence also 10 and 20 picks: their planes fill N 32 and
-// 64, whose groups pack a buffer without gaps (16 and 32 picks, N 48 and 96, took two and four buffers a row block and K step
-// where these take one and two). The codes as int8 in shared memory instead of tensor memory made 114 KB of shared-memory
-// traffic per step, 890 clocks.
+//   producer warp     per K step (256 codes = 4 groups): one bulk copy with the planes of the chunk's picks (8 KB per eight picks,
+//                     consecutive in memory and laid out as the operand wants them), then per row block the packed codes of 128
+//                     rows (128 bytes each, through a 3-D tensor map [expert][row][byte], 128-byte swizzle). Rings: 2 x 3 x 16 KB of
+//                     codes, 2 x 32 KB of planes
+//   2 table warps     the picks' scales, group sums and output rows of the next unit, and per two K steps the scales and minima of
+//                     the 256 rows (16 bytes each, cp.async) into a third ring
+//   8 converter warps thread = weight row = TMEM lane: the codes of half a K step -> fp16 straight into tensor memory (tcgen05.st,
+//                     one of four buffers of 64 columns), where tcgen05.mma takes its A operand from. Four warps take the first
+//                     half of every step, four the second: one set alone takes about as long as the copy of the codes
+//   MMA warp          per half step two groups of four tcgen05.mma (kind::f16, M 128, N 32 or 64, K 16) into columns of their own,
+//                     and one commit, which tells the converters that the code buffer is free and the epilogue that the sums are there
+//                     (the barrier cannot run two uses ahead of either: the products of its next use wait for both)
+//   16 epilogue warps thread = weight row = TMEM lane, four warps to a lane quarter, eight picks of both row blocks each: tcgen05.ld of
+//                     two groups, planes joined, times the row's group scale, plus the group minimum times the pick's group sum, group
+//                     after group: a pick's sum has this one order in chunks of every size (k_delta_prompt's note says why that
+//                     matters). Then activation scale and silu(gate) * up, or the picks' output rows
+//
+// What bounds it, per row block and K step (16 KB of codes, 2 KB of scales: 780 clocks of HBM at the SM's share): sixteen products,
+// which take 44 clocks each for any N up to 80, and commits, which take one product's time; about 850 clocks. So a chunk of 32 picks
+// costs what one pick costs, and eight picks (16 columns: eight of plane h, then eight of plane l) are the step by which lists grow.
 //
 // Every wait is a bounded mbarrier wait; a thread whose wait gave up skips its later waits, the producer stops issuing
 // copies and drains those in flight, and the kernel ends normally with the error word set.
@@ -44,33 +44,37 @@
 
 namespace b2 {
 
-constexpr int UQ_SMALL = 10;                     // picks of a small chunk: 30 of 32 accumulator columns per group
-constexpr int UQ_FEW = 4;                        // a chunk of at most this many (most experts of a step of up to 64 tokens): an epilogue warp takes two
-                                                 // picks, reads all four groups at once, and gives the buffer back before it folds them
-constexpr int UQ_TT = 20;                        // most picks per unit (a chunk of the pick list): 60 of 64 columns
-constexpr int UQ_WP = 5;                         // picks of an epilogue warp otherwise
-constexpr int UQ_XS = 6 * UQ_TT / UQ_WP;         // a group's pick sums: five, and one to keep the next five 8-byte aligned
-constexpr int UQ_KB = 256;                       // codes per K step: two 128-byte-wide sub-tiles, four groups
+constexpr int UQ_G = 8;                          // picks whose planes lie together: 16 accumulator columns per group
+constexpr int UQ_FEW = 8;                         // a chunk of at most this many picks has 16 accumulator columns per group, a buffer of 64 for a whole K step;
+constexpr int UQ_SMALL = 16;                     // picks of a small chunk: 32 columns per group, four accumulator buffers of half a K step
+constexpr int UQ_TT = 32;                        // most picks per unit (a chunk of the pick list): 64 columns, two buffers
+constexpr int UQ_KB = 256;                       // codes per K step: four groups
 constexpr int UQ_RAW = UM_M * UQ_KB / 2;         // 16 KB: packed codes of a row block and K step
-constexpr int UQ_BOX = 32;                       // plane rows per tensor copy
-constexpr int UQ_BSUB = UQ_BOX * UM_BK;          // 4 KB
-constexpr int UQ_PSLOT = 2 * 2 * UQ_BSUB;        // 16 KB: the planes of a K step
-constexpr int UQ_NW = 5, UQ_NP = 4, UQ_NS = 6;   // ring slots: codes, planes, row scales
-constexpr int UQ_SSLOT = 4 * UM_M * 8;           // 4 KB: [row block][scale | min][128 rows][4 groups] fp16 of a K step
-constexpr int UQ_RED = 2 * UQ_TT * UM_M * 4;     // 20 KB: a unit's sums, [row block][pick][row]
-constexpr int UQ_NA = 4;                         // code buffers in tensor memory
-constexpr int UQ_NACC = 2, UQ_ACC = 128;         // accumulator buffers, columns of each. A group's columns start at a multiple of N: a
-                                                 // tcgen05.mma whose accumulator does not start on the next power of two above N takes about three times as long
-constexpr int UQ_ACOL = UQ_NACC * UQ_ACC;        // the code buffers: 64 columns each (256 codes, 4 per 32-bit cell)
-constexpr int UQ_EPI = 16;                       // epilogue warps
-constexpr int UQ_THREADS = (8 + UQ_EPI) * 32;    // producer, MMA, 2 table warps, 4 converter warps, the epilogue
-constexpr size_t UQ_SMEM = (size_t)UQ_NW * UQ_RAW + (size_t)UQ_NP * UQ_PSLOT + (size_t)UQ_NS * UQ_SSLOT + UQ_RED + 1024;
+constexpr int UQ_PL = 2;                         // fp16 planes
+constexpr int UQ_GBYTES = UQ_G * UQ_PL * UQ_KB * 2;      // 8 KB: the planes of eight picks and a K step, [plane][group][pick][64 values]
+constexpr int UQ_SBO = UQ_KB / 64 * 1024;        // bytes between the eight rows of plane h, those of plane l, those of the next eight picks
+constexpr int UQ_PSLOT = UQ_TT / UQ_G * UQ_GBYTES;       // 32 KB
+constexpr int UQ_NW = 3, UQ_NP = 2, UQ_NS = 3;   // ring slots: codes of each row block, planes, row scales
+constexpr int UQ_SSLOT = 4 * UM_M * 16;          // 8 KB: [row block][scale | min][128 rows][8 groups] fp16 of two K steps
 constexpr int UQ_MAXG = 32;                      // groups of a row (K <= 2048)
+constexpr int UQ_XS = UQ_TT * UQ_MAXG * 4;       // 4 KB: a unit's group sums, [eight picks][group][pick]
+constexpr int UQ_RED = UQ_TT * UM_M * 4;         // 16 KB: the gate or up values that a warp hands to the one that finishes the pick, [pick][row]
+constexpr int UQ_NA = 4;                         // code buffers in tensor memory, 64 columns each (128 codes)
+constexpr int UQ_ACOL = 256;                     // where they start; the accumulators lie before them. A group's columns start at a multiple of N: a
+                                                 // tcgen05.mma whose accumulator does not start on the next power of two above N takes about three times as long
+constexpr int UQ_UNITS = 32;                     // units of a block whose places in the lists are looked up once
+constexpr int UQ_EPI = 8, UQ_CONV = 8;           // epilogue warps, converter warps
+constexpr int UQ_THREADS = (4 + UQ_CONV + UQ_EPI) * 32;  // producer, 2 MMA issuers, tables, converters, epilogue
+// Registers: the block is launched with 96 a thread; producer, issuers, tables and converters (three warpgroups) keep 64 and the epilogue's two
+// get 144: a buffer of 64 columns, the sums of 32 picks and what a fold needs. 3 x 64 + 2 x 144 = 5 x 96
+constexpr int UQ_REGS = 96, UQ_REGS_LOW = 64, UQ_REGS_EPI = 144;
+static_assert(UQ_REGS_LOW * (4 + UQ_CONV) + UQ_REGS_EPI * UQ_EPI <= UQ_REGS * (4 + UQ_CONV + UQ_EPI), "what the epilogue takes has been given back");
+constexpr size_t UQ_SMEM = (size_t)2 * UQ_NW * UQ_RAW + (size_t)UQ_NP * UQ_PSLOT + (size_t)UQ_NS * UQ_SSLOT + 2 * UQ_XS + UQ_RED + 1024;
 
 struct UmmaQ4Args {
-    CUtensorMap wmap;         // this matrix's packed codes of the layer's experts: [expert][row][K / 2 bytes], box 128 B x 64 rows
-    CUtensorMap xmap;         // planes [K / 128][slots][3][128 bytes] as rows of 128 bytes; box 32 rows (UQ_BOX), 128-byte swizzle
+    CUtensorMap wmap;         // this matrix's packed codes of the layer's experts: [expert][row][K / 2 bytes], box 128 B x 128 rows
     unsigned long long* trace;
+    const uint8_t* planes;    // [K step][slots / 8][UQ_GBYTES], the 16-byte pieces of a row where the 128-byte swizzle wants them
     const uint8_t* const* eptr;   // [E] expert blobs (for the scale and min rows)
     const int* list;          // pick ids sorted by expert (k_group_picks)
     ChunkTable small, big;    // chunks of at most UQ_SMALL picks, and of more
@@ -78,21 +82,22 @@ struct UmmaQ4Args {
     int up_row0;
     int e0;                   // first expert that lives on this GPU (its blob is index 0 of the tensor map)
     size_t off_s, off_m;      // the matrix's scale and min sections inside an expert blob
-    int slots;                // capacity of the planes (rows per plane)
+    int wide;                 // 16 bytes of a scale row (two K steps) may be copied at once
+    int slots;                // capacity of the planes
     const float* xscale;      // [slots] scale of each slot's planes
-    const float* xsum;        // [slots][K / 64] sum of each 64-value group of the slot's activations, in units of its scale
+    const float* xsum;        // [slots / 8][K / 64][8] sum of each 64-value group of the slots' activations, in units of their scale
     float* out;               // pair: act [picks][rows]; else ypart [tokens][topk + 1][rows]
     int* err;
 };
 
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-                 "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+                 "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
                  : "memory");
 }
 // D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void umma_i8_ts(uint32_t d, uint32_t atmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(atmem),
+__device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t atmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(atmem),
                  "l"(bdesc), "r"(idesc), "r"(accumulate)
                  : "memory");
 }
@@ -102,402 +107,455 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16]
                  "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(addr)
                  : "memory");
 }
-// 8 consecutive 32-bit columns of this thread's TMEM lane
-__device__ __forceinline__ void tmem_ld8(uint32_t addr, uint32_t (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+// one arrival when this thread's cp.async copies so far have landed
+__device__ __forceinline__ void mbar_arrive_copies(uint32_t bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_8(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+// 64 consecutive columns of this thread's TMEM lane, landed
+__device__ __forceinline__ void tmem_ld64(uint32_t addr, uint32_t (&r)[64]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x64.b32 {"
+                 "%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+                 "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,"
+                 "%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,"
+                 "%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%64];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+                   "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
+                   "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]), "=r"(r[33]),
+                   "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]),
+                   "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]),
+                   "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
                  : "r"(addr)
                  : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
-}
-// A pick's sum of one group. Columns 3 t + p hold plane p of pick t. The three plane sums are below 2^17 in
-// magnitude (64 codes of at most 15 times digits of at most 127), so d0 2^14 + d1 2^7 + d2 fits an int; 2^-14 is in the scale.
-template <int N>
-__device__ __forceinline__ float uq_value(const uint32_t (&c)[N], int t) {
-    return (float)((int)c[3 * t] * 16384 + ((int)c[3 * t + 1] * 128 + (int)c[3 * t + 2]));
-}
-// One group of 2 PAIRS (+ 1 with ONE) picks into their fp32 sums.
-template <int PAIRS, bool ONE, int N>
-__device__ __forceinline__ void uq_fold(const uint32_t (&c)[N], float sc, float mn, const float* xs, uint64_t (&acc)[2], float& acc1) {
-    const uint64_t sc2 = f2_pack(sc, sc), mn2 = f2_pack(mn, mn);
+// One group of eight picks into their fp32 sums: columns AT .. AT + 7 hold plane h of the picks, the next eight plane l, both in units of 2^-24; 2^-14 and
+// 2^24 are in the scale.
+template <int AT>
+__device__ __forceinline__ void uq_fold(const uint32_t (&c)[64], float sc, float mn, const float* xs, uint64_t (&acc)[4]) {
+    const uint64_t sc2 = f2_pack(sc, sc), mn2 = f2_pack(mn, mn), up = f2_pack(2048.0f, 2048.0f);
+    const ulonglong2 x0 = reinterpret_cast<const ulonglong2*>(xs)[0], x1 = reinterpret_cast<const ulonglong2*>(xs)[1];
+    const uint64_t x[4] = {x0.x, x0.y, x1.x, x1.y};
 #pragma unroll
-    for (int i = 0; i < PAIRS; i++)
-        acc[i] = f2_fma(sc2, f2_pack(uq_value(c, 2 * i), uq_value(c, 2 * i + 1)), f2_fma(mn2, reinterpret_cast<const uint64_t*>(xs)[i], acc[i]));
-    if (ONE) acc1 = fmaf(sc, uq_value(c, 2 * PAIRS), fmaf(mn, xs[2 * PAIRS], acc1));
+    for (int i = 0; i < 4; i++) {
+        const uint64_t h = f2_pack(__uint_as_float(c[AT + 2 * i]), __uint_as_float(c[AT + 2 * i + 1])),
+                       l = f2_pack(__uint_as_float(c[AT + 8 + 2 * i]), __uint_as_float(c[AT + 9 + 2 * i]));
+        acc[i] = f2_fma(sc2, f2_fma(h, up, l), f2_fma(mn2, x[i], acc[i]));
+    }
 }
 
-// The products of one accumulator buffer: all four groups of up to 10 picks (NT 1), or groups 2 turn and 2 turn + 1 of up to 20
-// (NT 2). Everything but the bases is a constant: with the groups, their column stride and N as run-time values the issuing
-// thread spent 160 to 200 clocks on each instruction (the tensor core needs about 44), and the whole kernel ran at that rate.
-template <int NT>
-__device__ __forceinline__ void uq_issue(uint32_t d, uint32_t at, uint64_t bd, int turn) {
-    constexpr uint32_t idesc = umma_idesc(2, 1, UM_M, NT * UQ_BOX);
-    constexpr int TG = 4 / NT;
+// The products of a group of 64 codes, N columns. Everything but the bases is a constant: with the groups, their column stride and N as
+// run-time values the issuing thread spent 160 to 200 clocks on each instruction.
+template <int N>
+__device__ __forceinline__ void uq_issue(uint32_t d, uint32_t at, uint64_t bd) {
+    constexpr uint32_t idesc = umma_idesc(1, 0, UM_M, N);
 #pragma unroll
-    for (int g = 0; g < TG; g++)
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int gg = turn * TG + g;
-            umma_i8_ts(d + g * NT * UQ_BOX, at + 16 * gg + 8 * k, bd + (uint64_t)((gg >> 1) * (NT * UQ_BSUB >> 4) + 4 * (gg & 1) + 2 * k), idesc, (uint32_t)k);
-        }
+    for (int k = 0; k < 4; k++) umma_f16_ts(d, at + 8 * k, bd + (uint64_t)(2 * k), idesc, (uint32_t)(k != 0));
 }
 
 __global__ void __launch_bounds__(UQ_THREADS, 1) k_umma_q4(const __grid_constant__ UmmaQ4Args a) {
     extern __shared__ unsigned char uq_raw[];
-    __shared__ __align__(8) uint64_t w_full[UQ_NW], w_empty[UQ_NW], p_full[UQ_NP], p_empty[UQ_NP], s_full[UQ_NS], s_empty[UQ_NS], t_full[2], t_empty[2], conv_bar[UQ_NA], a_empty[UQ_NA], acc_full[UQ_NACC], acc_empty[UQ_NACC];
+    // Code buffer and accumulator buffer 2 rb + h belong to row block rb. done[b]: the products that read code buffer b are over
+    // (first[b]: those of its first group); few[b]: accumulator buffer b holds a K step of few picks. A barrier never runs two phases ahead of
+    // a waiting warp: the products of its next phase need a code or accumulator buffer that the warp gives back only after this one (a K step
+    // of few picks, which needs one for both halves, sees to it itself)
+    enum { W_FULL = 0, W_EMPTY = W_FULL + 2 * UQ_NW, P_FULL = W_EMPTY + 2 * UQ_NW, P_EMPTY = P_FULL + UQ_NP, S_FULL = P_EMPTY + UQ_NP, S_EMPTY = S_FULL + UQ_NS, T_FULL = S_EMPTY + UQ_NS,
+           T_EMPTY = T_FULL + 2, CONV = T_EMPTY + 2, FIRST = CONV + UQ_NA, DONE = FIRST + UQ_NA, FEW = DONE + UQ_NA, ACC_EMPTY = FEW + UQ_NA, DRAINED = ACC_EMPTY + UQ_NA, NBAR };
+    __shared__ __align__(8) uint64_t s_bar[NBAR];
     __shared__ uint32_t tmem_slot;
-    __shared__ __align__(16) float s_xsum[2][UQ_MAXG][UQ_XS];      // group sums; the unit's and the next unit's
-    __shared__ float s_xscale[2][UQ_TT];
-    __shared__ int s_dst[2][UQ_TT];                  // output row index of each pick of the chunk (-1: not a pick)
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ __align__(16) float s_xscale[2][UQ_TT];
+    __shared__ __align__(16) int s_dst[2][UQ_TT];                  // where the output row of each pick of the chunk starts
+    __shared__ int4 s_unit[UQ_UNITS];                // the block's first units: expert, start, picks, first row
+    const int warp = threadIdx.x >> 5, lane = (int)held(threadIdx.x & 31);
     unsigned char* wring = uq_raw + ((1024u - (smem_u32(uq_raw) & 1023u)) & 1023u);
-    unsigned char* pring = wring + (size_t)UQ_NW * UQ_RAW;
+    unsigned char* pring = wring + (size_t)2 * UQ_NW * UQ_RAW;
     unsigned char* sring = pring + (size_t)UQ_NP * UQ_PSLOT;
-    float* red = reinterpret_cast<float*>(sring + (size_t)UQ_NS * UQ_SSLOT);
+    unsigned char* xsums = sring + (size_t)UQ_NS * UQ_SSLOT;
+    float* red = reinterpret_cast<float*>(xsums + 2 * UQ_XS);
     grid_dep_launch();
     trace_in(a.trace, 16, gridDim.x);
     if (threadIdx.x == 0) {
-        for (int s = 0; s < UQ_NW; s++) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], 4); }
-        for (int s = 0; s < UQ_NP; s++) { mbar_init(&p_full[s], 1); mbar_init(&p_empty[s], 1); }
-        for (int b = 0; b < UQ_NA; b++) { mbar_init(&conv_bar[b], 4); mbar_init(&a_empty[b], 1); }
-        for (int s = 0; s < UQ_NS; s++) { mbar_init(&s_full[s], 64); mbar_init(&s_empty[s], UQ_EPI); }
-        for (int b = 0; b < 2; b++) { mbar_init(&t_full[b], 64); mbar_init(&t_empty[b], UQ_EPI); }
-        for (int b = 0; b < UQ_NACC; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], UQ_EPI); }
+        auto init = [&](int first, int n, int count) { for (int i = 0; i < n; i++) mbar_init(&s_bar[first + i], count); };
+        init(W_FULL, 2 * UQ_NW, 1); init(W_EMPTY, 2 * UQ_NW, 4);
+        init(P_FULL, UQ_NP, 1); init(P_EMPTY, UQ_NP, 2);
+        init(S_FULL, UQ_NS, 32); init(S_EMPTY, UQ_NS, UQ_EPI);
+        init(T_FULL, 2, 32); init(T_EMPTY, 2, UQ_EPI);
+        init(CONV, UQ_NA, 4); init(FIRST, UQ_NA, 1); init(DONE, UQ_NA, 1); init(FEW, UQ_NA, 1); init(ACC_EMPTY, UQ_NA, 4);
+        init(DRAINED, 1, 2);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) tmem_alloc(&tmem_slot, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = held(tmem_slot);
+    const uint32_t bars = held(smem_u32(s_bar)), ring0 = held(smem_u32(wring));       // shared-memory addresses of the barriers and the rings
+    auto bar = [&](int kind, int i) { return bars + 8u * (uint32_t)(kind + i); };
     grid_dep_wait();                                 // the chunk tables, the planes and the activations are earlier launches' results
 
     const int nbig = *a.big.count, nsmall = *a.small.count;
     const int RG = a.pair ? a.rows / UM_M : a.rows / (2 * UM_M);      // units per chunk
-    const int nwork = (nbig + nsmall) * RG;          // big chunks first: they are the long ones
+    const int nwork = (nbig + nsmall) * RG;          // big chunks first
     const int nk = a.K / UQ_KB;                      // K steps per unit
     const int ngroup = a.K >> 6;
-    auto chunk_of = [&](int w, int& e, int& start, int& n, int& r0) {      // r0: the first weight row of the unit's first block
+    auto find = [&](int w) {
         const int c = w / RG;
-        r0 = (w - c * RG) * (a.pair ? UM_M : 2 * UM_M);
         const ChunkTable& t = c < nbig ? a.big : a.small;
         const int i = c < nbig ? c : c - nbig;
-        e = t.expert[i]; start = t.start[i]; n = t.n[i];
+        return make_int4(t.expert[i], t.start[i], t.n[i], (w - c * RG) * (a.pair ? UM_M : 2 * UM_M));
+    };
+    for (int i = threadIdx.x; i < UQ_UNITS && (int)(blockIdx.x + i * gridDim.x) < nwork; i += UQ_THREADS) s_unit[i] = find(blockIdx.x + i * gridDim.x);
+    __syncthreads();
+    // r0: the first weight row of the unit's first block. Every role asks once a unit; a table read costs a trip to L2 each time
+    auto chunk_of = [&](int w, int u, int& e, int& start, int& n, int& r0) {
+        const int4 v = u < UQ_UNITS ? s_unit[u] : find(w);
+        e = v.x; start = v.y; n = v.z; r0 = v.w;
     };
     const int rstep = a.pair ? a.up_row0 : UM_M;     // from the first row block to the second
-    auto wait = [&](uint64_t* bar, uint32_t parity, bool& dead) {
+    // bounded waits of a whole warp; one that gave up skips the rest
+    auto wait = [&](uint32_t at, uint32_t parity, bool& dead) {
         if (dead) return;
-        if (!mbar_wait(bar, parity, a.err, 1 << 21)) dead = true;
+        __syncwarp();
+        dead = !mbar_wait(at, parity, a.err, 1 << 21);
+        __syncwarp();
     };
 
-    if (warp < 8) {
+    if (warp < 4) regs_dec<UQ_REGS_LOW>();
     if (warp == 0) {
-        // ---- producer: one lane ----
-        if (lane == 0) {
-            int ws = 0, wph = 0, ps = 0, pph = 0;
-            bool dead = false;
-            uint32_t w_armed = 0, w_par = 0, p_armed = 0, p_par = 0;
-            for (int w = blockIdx.x; w < nwork && !dead; w += gridDim.x) {
-                int e, start, n, r0;
-                chunk_of(w, e, start, n, r0);
-                const int nt = n > UQ_SMALL ? 2 : 1;
-                for (int kc = 0; kc < nk && !dead; kc++) {
-                    wait(&p_empty[ps], pph ^ 1, dead);
-                    if (dead) break;
-                    mbar_expect_tx(&p_full[ps], (uint32_t)(2 * nt * UQ_BSUB));
-                    for (int s = 0; s < 2; s++)
-                        for (int j = 0; j < nt; j++)
-                            tma_load_2d(pring + (size_t)ps * UQ_PSLOT + (s * nt + j) * UQ_BSUB, &a.xmap, 0, ((kc * 2 + s) * a.slots + start) * UM_PI + UQ_BOX * j, &p_full[ps]);
-                    p_armed |= 1u << ps;
-                    p_par = (p_par & ~(1u << ps)) | ((uint32_t)pph << ps);
-                    if (++ps == UQ_NP) { ps = 0; pph ^= 1; }
-                    for (int rb = 0; rb < 2; rb++) {
-                        wait(&w_empty[ws], wph ^ 1, dead);
-                        if (dead) break;
-                        mbar_expect_tx(&w_full[ws], UQ_RAW);
-                        for (int h = 0; h < 2; h++)
-                            tma_load_3d(wring + (size_t)ws * UQ_RAW + h * (UQ_RAW / 2), &a.wmap, kc * (UQ_KB / 2), r0 + rb * rstep + h * 64, e - a.e0, &w_full[ws]);
-                        w_armed |= 1u << ws;
-                        w_par = (w_par & ~(1u << ws)) | ((uint32_t)wph << ws);
-                        if (++ws == UQ_NW) { ws = 0; wph ^= 1; }
-                    }
+        // ---- producer ----
+        int ws = 0, wph = 0, ps = 0, pph = 0;
+        bool dead = false;
+        uint32_t w_armed = 0, w_par = 0, p_armed = 0, p_par = 0;
+        for (int w = blockIdx.x, u = 0; w < nwork && !dead; w += gridDim.x, u++) {
+            int e, start, n, r0;
+            chunk_of(w, u, e, start, n, r0);
+            const uint32_t bytes = (uint32_t)((n + UQ_G - 1) / UQ_G) * UQ_GBYTES;
+            for (int kc = 0; kc < nk && !dead; kc++) {
+                wait(bar(P_EMPTY, ps), pph ^ 1, dead);
+                if (dead) break;
+                if (lane == 0) {
+                    mbar_expect_tx(bar(P_FULL, ps), bytes);
+                    bulk_load(ring0 + (uint32_t)(2 * UQ_NW * UQ_RAW + ps * UQ_PSLOT), a.planes + ((size_t)kc * a.slots + start) * (UQ_GBYTES / UQ_G), bytes, bar(P_FULL, ps));
                 }
-            }
-            if (dead) {                              // copies still in flight must land before the block may leave
-                for (int i = 0; i < UQ_NW; i++)
-                    if (w_armed >> i & 1) mbar_wait(&w_full[i], (w_par >> i) & 1u, nullptr, 1 << 16);
-                for (int i = 0; i < UQ_NP; i++)
-                    if (p_armed >> i & 1) mbar_wait(&p_full[i], (p_par >> i) & 1u, nullptr, 1 << 16);
+                p_armed |= 1u << ps;
+                p_par = (p_par & ~(1u << ps)) | ((uint32_t)pph << ps);
+                if (++ps == UQ_NP) { ps = 0; pph ^= 1; }
+                for (int rb = 0; rb < 2; rb++) {
+                    const int slot = rb * UQ_NW + ws;
+                    wait(bar(W_EMPTY, slot), wph ^ 1, dead);
+                    if (dead) break;
+                    if (lane == 0) {
+                        mbar_expect_tx(bar(W_FULL, slot), UQ_RAW);
+                        tma_load_3d(ring0 + (uint32_t)(slot * UQ_RAW), &a.wmap, kc * (UQ_KB / 2), r0 + rb * rstep, e - a.e0, bar(W_FULL, slot));
+                    }
+                    w_armed |= 1u << slot;
+                    w_par = (w_par & ~(1u << slot)) | ((uint32_t)wph << slot);
+                }
+                if (++ws == UQ_NW) { ws = 0; wph ^= 1; }
             }
         }
-    } else if (warp == 1) {
-        // ---- MMA issuer ----
-        if (elect_one()) {
-            int ps = 0, pph = 0, n = 0, tb = 0, tph = 0;       // n: (K step, row block) pairs so far; tb, tph: accumulator buffer and its use's parity
-            bool dead = false;
-            auto turns = [&](auto nt_, uint32_t at, uint64_t bd) {
-                constexpr int NT = decltype(nt_)::value;
-#pragma unroll
-                for (int t = 0; t < NT; t++) {
-                    wait(&acc_empty[tb], tph ^ 1, dead);       // the epilogue has read this buffer
-                    tc_fence_after();
-                    uq_issue<NT>(tmem + (uint32_t)tb * UQ_ACC, at, bd, t);
-                    umma_commit(&acc_full[tb]);
-                    if (++tb == UQ_NACC) { tb = 0; tph ^= 1; }
-                }
-            };
-            for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
-                int e, start, cn, r0;
-                chunk_of(w, e, start, cn, r0);
-                for (int kc = 0; kc < nk; kc++) {
-                    wait(&p_full[ps], pph, dead);
-                    const uint64_t bd = umma_desc_sw128(smem_u32(pring + (size_t)ps * UQ_PSLOT));
-                    for (int rb = 0; rb < 2; rb++, n++) {
-                        const int buf = n & (UQ_NA - 1);
-                        wait(&conv_bar[buf], (n / UQ_NA) & 1, dead);
-                        tc_fence_after();
-                        const uint32_t at = tmem + UQ_ACOL + 64u * buf;
-                        if (cn > UQ_SMALL) turns(UqInt<2>(), at, bd); else turns(UqInt<1>(), at, bd);
-                        umma_commit(&a_empty[buf]);
-                    }
-                    umma_commit(&p_empty[ps]);
-                    if (++ps == UQ_NP) { ps = 0; pph ^= 1; }
-                }
-            }
+        if (dead && lane == 0) {                     // copies still in flight must land before the block may leave
+            for (int i = 0; i < 2 * UQ_NW; i++)
+                if (w_armed >> i & 1) mbar_wait(bar(W_FULL, i), (w_par >> i) & 1u, nullptr, 1 << 16);
+            for (int i = 0; i < UQ_NP; i++)
+                if (p_armed >> i & 1) mbar_wait(bar(P_FULL, i), (p_par >> i) & 1u, nullptr, 1 << 16);
         }
         __syncwarp();
-    } else if (warp < 4) {
-        // ---- tables: 64 threads ----
-        const int tt = threadIdx.x - 64;
-        int u = 0, st = 0, ph = 0;
-        bool dead = false;
-        // rows tt and tt + 64 of (row block, scale | min): address of a unit's first K step
-        const uint8_t *bs = nullptr, *bm = nullptr;
-        size_t row_off = 0;
-        const size_t half = (size_t)64 * ngroup * 2, rbs = (size_t)rstep * ngroup * 2;
-        auto locate = [&](int w, int& start, int& cn) {
-            int e, r0;
-            chunk_of(w, e, start, cn, r0);
-            const uint8_t* blob = a.eptr[e];
-            bs = blob + a.off_s; bm = blob + a.off_m;
-            row_off = (size_t)(r0 + tt) * ngroup * 2;
-        };
-        auto src = [&](int i) { return (i & 2 ? bm : bs) + row_off + (i & 1 ? half : 0) + (i & 4 ? rbs : 0); };
-        uint2 v[8];
-        int start, cn;
-        if ((int)blockIdx.x < nwork) {
-            locate(blockIdx.x, start, cn);
-#pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = *reinterpret_cast<const uint2*>(src(i));
-        }
-        for (int w = blockIdx.x; w < nwork; w += gridDim.x, u++) {
-            const int ub = u & 1;
-            wait(&t_empty[ub], ((u >> 1) & 1) ^ 1, dead);
-            if (tt < UQ_TT) {
-                const int p = tt < cn ? a.list[start + tt] : -1;
-                s_xscale[ub][tt] = tt < cn ? a.xscale[start + tt] : 0.f;
-                s_dst[ub][tt] = p >= 0 ? (a.pair ? p : (p / a.topk) * (a.topk + 1) + p % a.topk) : -1;
-            }
-            for (int i = tt; i < UQ_TT * ngroup; i += 64) {
-                const int t = i / ngroup, g = i - t * ngroup;
-                s_xsum[ub][g][t + t / UQ_WP] = t < cn ? a.xsum[(size_t)(start + t) * ngroup + g] : 0.f;
-            }
-            mbar_arrive(&t_full[ub]);
-            for (int kc = 0; kc < nk; kc++) {
-                // the step's values are in registers or on their way; the next step's (of the next unit after the last) are asked
-                // for before these are stored, the next unit's rows brought towards L2 at the unit's first step
-                uint2 n[8];
-                if (kc + 1 < nk) {
-#pragma unroll
-                    for (int i = 0; i < 8; i++) n[i] = *reinterpret_cast<const uint2*>(src(i) + 8 * (kc + 1));
-                } else if (w + (int)gridDim.x < nwork) {
-                    locate(w + gridDim.x, start, cn);
-#pragma unroll
-                    for (int i = 0; i < 8; i++) n[i] = *reinterpret_cast<const uint2*>(src(i));
-                }
-                if (kc == 0 && nk > 1 && w + (int)gridDim.x < nwork) {
-                    int e2, s2, c2, r2;
-                    chunk_of(w + gridDim.x, e2, s2, c2, r2);
-                    const uint8_t* b = a.eptr[e2] + (size_t)(r2 + tt) * ngroup * 2;
-#pragma unroll
-                    for (int i = 0; i < 8; i++)
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(b + (i & 2 ? a.off_m : a.off_s) + (i & 1 ? half : 0) + (i & 4 ? rbs : 0)));
-                }
-                wait(&s_empty[st], ph ^ 1, dead);
-                uint2* dst = reinterpret_cast<uint2*>(sring + (size_t)st * UQ_SSLOT) + tt;
-#pragma unroll
-                for (int i = 0; i < 8; i++) dst[(i >> 1) * UM_M + 64 * (i & 1)] = v[i];
-                mbar_arrive(&s_full[st]);
-                if (++st == UQ_NS) { st = 0; ph ^= 1; }
-#pragma unroll
-                for (int i = 0; i < 8; i++) v[i] = n[i];
-            }
-        }
-    } else {
-        // ---- converters: this thread's row of 128 packed bytes -> 64 cells of four int8 codes in its TMEM lane ----
-        const int q = warp & 3, r = q * 32 + lane;
-        const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
-        int st = 0, ph = 0, n = 0;
-        bool dead = false;
-        const uint32_t never = (uint32_t)a.pair >> 1;        // 0 (pair is 0 or 1)
-        for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
-            for (int step = 0; step < 2 * nk; step++, n++) {
-                const int buf = n & (UQ_NA - 1);
-                wait(&w_full[st], ph, dead);
-                // rows of 128 bytes in two boxes of 64; the copy's 128-byte swizzle puts 16-byte piece c of row r at c ^ (r & 7), so
-                // the same piece of eight neighbouring rows covers all banks
-                const unsigned char* row = wring + (size_t)st * UQ_RAW + r * 128;
-                uint4 pk[8];
-#pragma unroll
-                for (int c = 0; c < 8; c++) pk[c] = *reinterpret_cast<const uint4*>(row + ((c ^ (r & 7)) << 4));
-                // The slot may be refilled once the codes are in registers, not once their loads are issued: with nothing that
-                // uses the values before the arrival they were seen to come from the slot's next contents, with the wait below
-                // in between. The address depends on one word of each load (none is a constant 0 the compiler could know). Lane 0's
-                // words stand for the warp's: a load is one instruction for all its lanes, and its result is waited for as a whole.
-                const uint32_t used = ((pk[0].x ^ pk[1].x) | (pk[2].x ^ pk[3].x) | (pk[4].x ^ pk[5].x) | (pk[6].x ^ pk[7].x)) & never;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&w_empty[st] + used);
-                if (++st == UQ_NW) { st = 0; ph ^= 1; }
-                wait(&a_empty[buf], ((n / UQ_NA) & 1) ^ 1, dead);              // the MMAs that read this code buffer are done
-                __syncwarp();
-                tc_fence_after();
-#pragma unroll
-                for (int c = 0; c < 8; c += 2) {
-                    // the eight codes of a word as even ones, then odd ones: the planes hold their values in the same order
-                    const uint32_t pw[8] = {pk[c].x, pk[c].y, pk[c].z, pk[c].w, pk[c + 1].x, pk[c + 1].y, pk[c + 1].z, pk[c + 1].w};
-                    uint32_t o[16];
-#pragma unroll
-                    for (int i = 0; i < 8; i++) { o[2 * i] = pw[i] & 0x0F0F0F0Fu; o[2 * i + 1] = (pw[i] >> 4) & 0x0F0F0F0Fu; }
-                    tmem_st16(tmem + lane_addr + UQ_ACOL + 64u * buf + 8u * c, o);
-                }
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&conv_bar[buf]);
-            }
-        }
-    }
-    } else {
-        // ---- epilogue: warp w may touch TMEM lanes 32 (w % 4) .. + 31 ----
-        const int q = warp & 3, j = (warp - 8) >> 2, set = j & 1, half = j >> 1;
-        const int vrow = q * 32 + lane;
-        const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
-        int par = 0, u = 0, st = 0, ph = 0;          // bit b: parity of accumulator buffer b's use; units so far; scale slot and its parity
-        bool dead = false;
-        for (int w = blockIdx.x; w < nwork; w += gridDim.x, u++) {
+    } else if (warp < 3) {
+        // ---- MMA issuers, one for each row block: a warp waits, its elected lane issues ----
+        const int rb = warp - 1;
+        int ps = 0, pph = 0;
+        uint32_t kg = 0, turn = 0, dk = 0;           // K steps and uses of an accumulator buffer so far
+        const uint32_t d0 = tmem + 128u * rb;
+        bool dead = false, was_few = false;
+        const bool lead = elect_one();
+        for (int w = blockIdx.x, u = 0; w < nwork; w += gridDim.x, u++) {
             int e, start, cn, r0;
-            chunk_of(w, e, start, cn, r0);
-            const int ub = u & 1;
-            wait(&t_full[ub], (u >> 1) & 1, dead);
-            // A small chunk's buffer is a (K step, row block) pair with all four groups: the number of buffers before a unit is even, so
-            // buffer 0 gets the first row block and buffer 1 the second; set 0 takes the first, set 1 the second, a warp half of the
-            // picks. A larger chunk's pair is two buffers of two groups each: every warp reads both, five picks each. The
-            // loops stay rolled, with the row blocks' sums changing places instead: the bodies of all roles run at the same time, and where a
-            // body does not fit the schedulers' instruction caches the warps wait for instructions (450 instructions: 31 clocks a value)
-            uint64_t acc[2][2];                      // [row block (a small chunk: only the first)][pick pairs]
-            float acc1[2] = {0.f, 0.f};              // and the fifth pick
-            acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = 0ull;
+            chunk_of(w, u, e, start, cn, r0);
             const bool big = cn > UQ_SMALL, few = cn <= UQ_FEW;
-            const int p0 = big ? UQ_WP * j : (few ? 2 : UQ_WP) * half;           // this warp's first pick
-            const uint32_t cstep = big ? 64u : 32u;                              // columns between two groups
-            const uint32_t col0 = tmem + lane_addr + 3u * p0;
-            auto release = [&](int b) {              // the buffer is in registers: the next products may overwrite it
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_n(&acc_empty[b], big ? 1u : 2u);      // 16 warps, or 8 that count twice
-                par ^= 1 << b;
-            };
+            bool catch_up = few && !was_few;         // see below
+            was_few = few;
+            for (int kc = 0; kc < nk; kc++, kg++) {
+                wait(bar(P_FULL, ps), pph, dead);
+                const uint64_t bd = (umma_desc_sw128(ring0 + (uint32_t)(2 * UQ_NW * UQ_RAW + ps * UQ_PSLOT)) & ~(0x3FFFull << 32)) | ((uint64_t)(UQ_SBO >> 4) << 32);
 #pragma unroll 1
-            for (int kc = 0; kc < nk; kc++) {
-                wait(&s_full[st], ph, dead);
-                const uint2* sc4 = reinterpret_cast<const uint2*>(sring + (size_t)st * UQ_SSLOT) + vrow;
-                const float* xs = &s_xsum[ub][4 * kc][p0 + (few ? 0 : p0 / UQ_WP)];
-#pragma unroll 1
-                for (int rb = big ? 0 : set; rb < 2; rb += big ? 1 : 2) {
-                    const uint2 s4 = sc4[(2 * rb) * UM_M], m4 = sc4[(2 * rb + 1) * UM_M];
-                    if (few) {
-                        wait(&acc_full[set], (par >> set) & 1, dead);
-                        __syncwarp();                // tcgen05.ld needs the whole warp at once
+                for (int h = 0; h < 2; h++) {
+                    const int b = 2 * rb + h;
+                    const uint32_t at = tmem + UQ_ACOL + 64u * b;
+                    const uint64_t bh = bd + (uint64_t)(h * (2048 >> 4));
+                    wait(bar(CONV, b), kg & 1, dead);
+                    // the next accumulator buffer: for both groups of this half, for each, or (few picks) for the whole K step
+                    auto buffer = [&]() {
+                        const uint32_t i = turn & 1;
+                        wait(bar(ACC_EMPTY, 2 * rb + (int)i), ((turn >> 1) & 1) ^ 1, dead);
                         tc_fence_after();
-                        uint32_t c[4][8];
-#pragma unroll
-                        for (int g = 0; g < 4; g++) tmem_ld8(col0 + (uint32_t)set * UQ_ACC + 32u * g, c[g]);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int g = 0; g < 4; g++)
-#pragma unroll
-                            for (int i = 0; i < 6; i++) asm volatile("" : "+r"(c[g][i]));        // uses of the values stay behind the wait
-                        release(set);
-#pragma unroll
-                        for (int g = 0; g < 4; g++) {
-                            const uint32_t sw = g < 2 ? s4.x : s4.y, mw = g < 2 ? m4.x : m4.y;
-                            uq_fold<1, false>(c[g], h2f((uint16_t)(g & 1 ? sw >> 16 : sw & 0xFFFFu)) * (1.0f / 16384.0f),
-                                              h2f((uint16_t)(g & 1 ? mw >> 16 : mw & 0xFFFFu)), xs + g * UQ_XS, acc[0], acc1[0]);
+                        turn++;
+                        return d0 + 64u * i;
+                    };
+                    if (big) {
+                        uint32_t d = buffer();
+                        if (lead) { uq_issue<64>(d, at, bh); umma_commit(bar(FIRST, b)); }
+                        __syncwarp();
+                        d = buffer();
+                        if (lead) { uq_issue<64>(d, at + 32, bh + (1024 >> 4)); umma_commit(bar(DONE, b)); }
+                    } else if (few) {
+                        // With one buffer for both halves these products could end a second phase of done[b] while the epilogue still waits for
+                        // the first, that of a larger chunk before this one: behind such a chunk its last buffer must have been read first
+                        if (h == 0) dk = buffer();
+                        else if (catch_up) { wait(bar(ACC_EMPTY, 2 * rb + (int)(turn & 1)), ((turn >> 1) & 1) ^ 1, dead); catch_up = false; }
+                        tc_fence_after();
+                        if (lead) {
+                            uq_issue<16>(dk + 32u * h, at, bh);
+                            uq_issue<16>(dk + 32u * h + 16, at + 32, bh + (1024 >> 4));
+                            umma_commit(bar(DONE, b));
+                            if (h) umma_commit(bar(FEW, 2 * rb + (int)((turn - 1) & 1)));
                         }
                     } else {
-#pragma unroll 1
-                        for (int h = 0; h < 2; h++) {                            // groups 2 h and 2 h + 1
-                            const int b = big ? h : set;
-                            if (big || h == 0) wait(&acc_full[b], (par >> b) & 1, dead);
-                            __syncwarp();
-                            tc_fence_after();
-                            const uint32_t col = col0 + (uint32_t)b * UQ_ACC + (big ? 0u : 64u * h);
-                            uint32_t c[2][16];
-                            tmem_ld16(col, c[0]);
-                            tmem_ld16(col + cstep, c[1]);
-                            tmem_ld_wait();
-#pragma unroll
-                            for (int i = 0; i < 15; i++) { asm volatile("" : "+r"(c[0][i])); asm volatile("" : "+r"(c[1][i])); }
-                            if (big || h) release(b);
-                            const uint32_t sw = h ? s4.y : s4.x, mw = h ? m4.y : m4.x;
-                            uq_fold<2, true>(c[0], h2f((uint16_t)(sw & 0xFFFFu)) * (1.0f / 16384.0f), h2f((uint16_t)(mw & 0xFFFFu)), xs + 2 * h * UQ_XS, acc[0], acc1[0]);
-                            uq_fold<2, true>(c[1], h2f((uint16_t)(sw >> 16)) * (1.0f / 16384.0f), h2f((uint16_t)(mw >> 16)), xs + (2 * h + 1) * UQ_XS, acc[0], acc1[0]);
+                        const uint32_t d = buffer();
+                        if (lead) {
+                            uq_issue<32>(d, at, bh);
+                            uq_issue<32>(d + 32, at + 32, bh + (1024 >> 4));
+                            umma_commit(bar(DONE, b));
                         }
                     }
-                    if (big) {
+                    __syncwarp();
+                }
+                if (lead) umma_commit(bar(P_EMPTY, ps));
+                __syncwarp();
+                if (++ps == UQ_NP) { ps = 0; pph ^= 1; }
+            }
+        }
+        if (lead) umma_commit(bar(DRAINED, 0));             // no product may be under way when the block gives its tensor memory back
+        __syncwarp();
+        mbar_wait(bar(DRAINED, 0), 0, a.err, 1 << 21);
+    } else if (warp == 3) {
+        // ---- tables ----
+        int u = 0, st = 0, ph = 0;
+        bool dead = false;
+        const size_t step = (size_t)32 * ngroup * 2, rbs = (size_t)rstep * ngroup * 2;
+        for (int w = blockIdx.x; w < nwork && !dead; w += gridDim.x, u++) {
+            const int ub = u & 1;
+            int e, start, cn, r0;
+            chunk_of(w, u, e, start, cn, r0);
+            wait(bar(T_EMPTY, ub), ((u >> 1) & 1) ^ 1, dead);
+            if (dead) break;
+            if (lane < cn) {
+                const int p = a.list[start + lane];
+                s_xscale[ub][lane] = a.xscale[start + lane];
+                s_dst[ub][lane] = (a.pair ? p : (p / a.topk) * (a.topk + 1) + p % a.topk) * a.rows;
+            }
+            if (lane == 0) {
+                const uint32_t bytes = (uint32_t)((cn + UQ_G - 1) / UQ_G * UQ_G * ngroup * 4);
+                mbar_expect_tx(bar(T_FULL, ub), bytes);
+                bulk_load(xsums + (size_t)ub * UQ_XS, a.xsum + (size_t)start * ngroup, bytes, bar(T_FULL, ub));
+            } else {
+                mbar_arrive(bar(T_FULL, ub));
+            }
+            const uint8_t* blob = a.eptr[e];
+            const size_t row_off = (size_t)(r0 + lane) * ngroup * 2;
+            for (int kc = 0; kc < nk; kc += 2) {
+                wait(bar(S_EMPTY, st), ph ^ 1, dead);
+                if (dead) break;
+                const uint32_t dst = ring0 + (uint32_t)(2 * UQ_NW * UQ_RAW + UQ_NP * UQ_PSLOT + st * UQ_SSLOT + lane * 16);
 #pragma unroll
-                        for (int i = 0; i < 2; i++) { const uint64_t v = acc[0][i]; acc[0][i] = acc[1][i]; acc[1][i] = v; }
-                        const float v = acc1[0];
-                        acc1[0] = acc1[1]; acc1[1] = v;
+                for (int i = 0; i < 16; i++) {       // rows lane, + 32, .. of (row block, scale | min)
+                    const uint8_t* src = blob + (i & 4 ? a.off_m : a.off_s) + row_off + (i & 3) * step + (i & 8 ? rbs : 0) + 8 * kc;
+                    const uint32_t d = dst + ((i >> 2) * UM_M + 32 * (i & 3)) * 16;
+                    if (a.wide) {
+                        cp_async_16(d, src);
+                    } else {
+                        cp_async_8(d, src);
+                        if (kc + 1 < nk) cp_async_8(d + 8, src + 8);
                     }
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&s_empty[st]);
+                mbar_arrive_copies(bar(S_FULL, st));
                 if (++st == UQ_NS) { st = 0; ph ^= 1; }
             }
-            // the other set's buffer had nk uses that this warp took no part in (all are over: the barrier below is behind both sets' last)
-            if (!big) par ^= (nk & 1) << (set ^ 1);
-            float* rd = red + vrow;
-            {
-                float* dst = rd + ((big ? 0 : set * UQ_TT) + p0) * UM_M;
-                f2_unpack(acc[0][0], dst[0], dst[UM_M]);
-                if (!few) { f2_unpack(acc[0][1], dst[2 * UM_M], dst[3 * UM_M]); dst[4 * UM_M] = acc1[0]; }
-                if (big) {
-                    dst += UQ_TT * UM_M;
-                    f2_unpack(acc[1][0], dst[0], dst[UM_M]);
-                    f2_unpack(acc[1][1], dst[2 * UM_M], dst[3 * UM_M]);
-                    dst[4 * UM_M] = acc1[1];
+        }
+        // copies still in flight must land before the block may leave
+        cp_async_commit();
+        cp_async_wait<0>();
+        if (lane == 0)
+            for (int i = u > 2 ? u - 2 : 0; i < u; i++) mbar_wait(bar(T_FULL, i & 1), (i >> 1) & 1, nullptr, 1 << 16);
+        __syncwarp();
+    } else if (warp < 4 + UQ_CONV) {
+        // ---- converters, four warps to a row block: this thread's row of 128 packed bytes -> 2 x 64 cells of two fp16 codes in its TMEM lane ----
+        regs_dec<UQ_REGS_LOW>();
+        const int q = warp & 3, rb = (warp >> 2) - 1, r = q * 32 + lane;
+        const uint32_t col0 = tmem + ((uint32_t)(q * 32) << 16) + UQ_ACOL + 128u * rb;
+        int st = 0, ph = 0;                          // a ring for each row block: shared, one's converters would pass a barrier by that the other's wait for
+        uint32_t kg = 0;
+        bool dead = false;
+        for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
+            for (int kc = 0; kc < nk; kc++, kg++) {
+                wait(bar(W_FULL, rb * UQ_NW + st), ph, dead);
+                const unsigned char* row = wring + (size_t)(rb * UQ_NW + st) * UQ_RAW + r * 128;
+#pragma unroll 1
+                for (int h = 0; h < 2; h++) {
+                    // the copy's 128-byte swizzle puts 16-byte piece c of row r at c ^ (r & 7), so the same piece of eight neighbouring rows covers all banks
+                    uint4 pk[4];
+#pragma unroll
+                    for (int c = 0; c < 4; c++) pk[c] = *reinterpret_cast<const uint4*>(row + (((4 * h + c) ^ (r & 7)) << 4));
+                    wait(bar(DONE, 2 * rb + h), (kg & 1) ^ 1, dead);                     // the products that read this code buffer are over
+                    tc_fence_after();
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        // eight codes of a word: 0 and 4, 1 and 5, 2 and 6, 3 and 7 to a cell; the planes hold their values in the same order
+                        const uint32_t pw[4] = {pk[c].x, pk[c].y, pk[c].z, pk[c].w};
+                        uint32_t o[16];
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            o[4 * i] = pw[i] & 0x000F000Fu; o[4 * i + 1] = pw[i] & 0x00F000F0u;
+                            o[4 * i + 2] = (pw[i] >> 8) & 0x000F000Fu; o[4 * i + 3] = (pw[i] >> 8) & 0x00F000F0u;
+                        }
+                        tmem_st16(col0 + 64u * h + 16u * c, o);
+                    }
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    tc_fence_before();
+                    __syncwarp();
+                    mbar_arrive_if(lane == 0, bar(CONV, 2 * rb + h));
                 }
+                // the stores have taken the codes out of the registers, so their loads have left the ring slot
+                mbar_arrive_if(lane == 0, bar(W_EMPTY, rb * UQ_NW + st));
+                if (++st == UQ_NW) { st = 0; ph ^= 1; }
             }
-            asm volatile("bar.sync %0, 128;" ::"r"(1 + q) : "memory");           // the quarter's four warps
-            // act = silu(gate) * up per pick (pairs), or the picks' rows of ypart (nothing after a wait that gave up: the tables may be stale)
-#pragma unroll 2
-            for (int t = j; t < (dead ? 0 : cn); t += 4) {
-                const float xsc = s_xscale[ub][t];
-                const float v0 = rd[t * UM_M] * xsc, v1 = rd[(UQ_TT + t) * UM_M] * xsc;
-                float* out = a.out + (size_t)s_dst[ub][t] * a.rows + r0 + vrow;
-                if (a.pair) {
-                    *out = siluf_(v0) * v1;
-                } else {
-                    out[0] = v0;
-                    out[UM_M] = v1;
-                }
-            }
-            asm volatile("bar.sync %0, 128;" ::"r"(1 + q) : "memory");           // all are through: the next unit may write its sums
+        }
+    } else {
+        // ---- epilogue: warp w may touch TMEM lanes 32 (w % 4) .. + 31; four warps to a row block ----
+        regs_inc<UQ_REGS_EPI>();
+        const int q = warp & 3, rb = (warp - 4 - UQ_CONV) >> 2;
+        const int vrow = q * 32 + lane;
+        const uint32_t col0 = held(tmem + ((uint32_t)(q * 32) << 16) + 128u * rb);
+        int st = 0, ph = 0;
+        uint32_t kg = 0, turn = 0, few_par = 0, first_par = 0;       // few_par: bit i, the parity of few[2 rb + i]'s next phase; first_par: of first's
+        bool dead = false;
+        uint32_t c[64];
+        // the next accumulator buffer into registers, once the products that `full` stands for are over; then they may overwrite it
+        auto load = [&](uint32_t full, uint32_t parity) {
+            wait(full, parity, dead);
+            tc_fence_after();
+            tmem_ld64(col0 + 64u * (turn & 1), c);
+            tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&t_empty[ub]);
+            mbar_arrive_if(lane == 0, bar(ACC_EMPTY, 2 * rb + (int)(turn & 1)));
+            turn++;
+        };
+        for (int w = blockIdx.x, u = 0; w < nwork; w += gridDim.x, u++) {
+            int e, start, cn, r0;
+            chunk_of(w, u, e, start, cn, r0);
+            const int ub = u & 1;
+            wait(bar(T_FULL, ub), (u >> 1) & 1, dead);
+            const float* xs = reinterpret_cast<const float*>(xsums + (size_t)ub * UQ_XS);
+            const int xg = ngroup * UQ_G;            // to the sums of the next eight picks
+            uint64_t acc[UQ_TT / UQ_G][4];
+#pragma unroll
+            for (int s = 0; s < UQ_TT / UQ_G; s++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) acc[s][i] = 0ull;
+#pragma unroll 1
+            for (int kc = 0; kc < nk; kc++, kg++, xs += 4 * UQ_G) {
+                if (!(kc & 1)) wait(bar(S_FULL, st), ph, dead);
+                const unsigned char* sc4 = sring + (size_t)st * UQ_SSLOT + (2 * rb * UM_M + vrow) * 16 + (kc & 1) * 8;
+                const uint2 s4 = *reinterpret_cast<const uint2*>(sc4), m4 = *reinterpret_cast<const uint2*>(sc4 + UM_M * 16);
+                if (cn <= UQ_FEW) {                  // a buffer holds the four groups of eight picks
+                    const uint32_t i = turn & 1;
+                    load(bar(FEW, 2 * rb + (int)i), (few_par >> i) & 1);
+                    few_par ^= 1u << i;
+                    uq_fold<0>(c, f16_of(s4.x, 0) * 1024.0f, f16_of(m4.x, 0), xs, acc[0]);
+                    uq_fold<16>(c, f16_of(s4.x, 1) * 1024.0f, f16_of(m4.x, 1), xs + UQ_G, acc[0]);
+                    uq_fold<32>(c, f16_of(s4.y, 0) * 1024.0f, f16_of(m4.y, 0), xs + 2 * UQ_G, acc[0]);
+                    uq_fold<48>(c, f16_of(s4.y, 1) * 1024.0f, f16_of(m4.y, 1), xs + 3 * UQ_G, acc[0]);
+                } else {
+                    const float* x = xs;
+#pragma unroll 1
+                    for (int h = 0; h < 2; h++, x += 2 * UQ_G) {
+                        const uint32_t sw = h ? s4.y : s4.x, mw = h ? m4.y : m4.x;
+                        const float sca = f16_of(sw, 0) * 1024.0f, scb = f16_of(sw, 1) * 1024.0f, mna = f16_of(mw, 0), mnb = f16_of(mw, 1);
+                        if (cn <= UQ_SMALL) {        // two groups of sixteen
+                            load(bar(DONE, 2 * rb + h), kg & 1);
+                            uq_fold<0>(c, sca, mna, x, acc[0]);
+                            uq_fold<16>(c, sca, mna, x + xg, acc[1]);
+                            uq_fold<32>(c, scb, mnb, x + UQ_G, acc[0]);
+                            uq_fold<48>(c, scb, mnb, x + xg + UQ_G, acc[1]);
+                        } else {                     // one group of 32
+#pragma unroll
+                            for (int g = 0; g < 2; g++) {
+                                load(g ? bar(DONE, 2 * rb + h) : bar(FIRST, 2 * rb + h), g ? kg & 1 : first_par);
+                                const float sc = g ? scb : sca, mn = g ? mnb : mna;
+                                const float* xx = x + g * UQ_G;
+                                uq_fold<0>(c, sc, mn, xx, acc[0]);
+                                uq_fold<16>(c, sc, mn, xx + xg, acc[1]);
+                                uq_fold<32>(c, sc, mn, xx + 2 * xg, acc[2]);
+                                uq_fold<48>(c, sc, mn, xx + 3 * xg, acc[3]);
+                            }
+                        }
+                    }
+                }
+                if (cn > UQ_SMALL) first_par ^= 1;
+                if ((kc & 1) || kc + 1 == nk) {
+                    __syncwarp();
+                    mbar_arrive_if(lane == 0, bar(S_EMPTY, st));
+                    if (++st == UQ_NS) { st = 0; ph ^= 1; }
+                }
+            }
+            // act = silu(gate) * up per pick (pairs): of every eight picks the gate rows' warp finishes the first four and the up rows' warp the
+            // others; or the picks' rows of ypart (nothing after a wait that gave up: the tables may be stale)
+            const int np = dead ? 0 : cn;
+            float* out = a.out + r0 + vrow;
+            if (a.pair) {
+                float* rd = red + (size_t)(rb ? 0 : 4) * UM_M + vrow;
+                asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");        // the unit before has read its values
+#pragma unroll
+                for (int s = 0; s < UQ_TT / UQ_G; s++) {
+                    if (UQ_G * s >= cn) break;
+                    f2_unpack(rb ? acc[s][0] : acc[s][2], rd[UQ_G * s * UM_M], rd[(UQ_G * s + 1) * UM_M]);
+                    f2_unpack(rb ? acc[s][1] : acc[s][3], rd[(UQ_G * s + 2) * UM_M], rd[(UQ_G * s + 3) * UM_M]);
+                }
+                asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");        // the quarter's two warps
+#pragma unroll
+                for (int s = 0; s < UQ_TT / UQ_G; s++) {
+                    const int t = UQ_G * s + 4 * rb;
+                    if (t >= np) break;
+                    const float4 x4 = *reinterpret_cast<const float4*>(&s_xscale[ub][t]);
+                    const int4 d4 = *reinterpret_cast<const int4*>(&s_dst[ub][t]);
+                    const float xsc[4] = {x4.x, x4.y, x4.z, x4.w};
+                    const int dst[4] = {d4.x, d4.y, d4.z, d4.w};
+                    float own[4];
+                    f2_unpack(rb ? acc[s][2] : acc[s][0], own[0], own[1]);
+                    f2_unpack(rb ? acc[s][3] : acc[s][1], own[2], own[3]);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const float o = red[(size_t)(t + i) * UM_M + vrow];
+                        const float y = siluf_((rb ? o : own[i]) * xsc[i]) * ((rb ? own[i] : o) * xsc[i]);
+                        if (t + i < np) out[dst[i]] = y;
+                    }
+                }
+            } else {
+                out += rb * UM_M;
+#pragma unroll
+                for (int t = 0; t < UQ_TT; t += 4) {
+                    if (t >= np) break;
+                    const float4 x4 = *reinterpret_cast<const float4*>(&s_xscale[ub][t]);
+                    const int4 d4 = *reinterpret_cast<const int4*>(&s_dst[ub][t]);
+                    const float xsc[4] = {x4.x, x4.y, x4.z, x4.w};
+                    const int dst[4] = {d4.x, d4.y, d4.z, d4.w};
+                    float v[4];
+                    f2_unpack(acc[t / UQ_G][(t & 4) / 2], v[0], v[1]);
+                    f2_unpack(acc[t / UQ_G][(t & 4) / 2 + 1], v[2], v[3]);
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        if (t + i < np) out[dst[i]] = v[i] * xsc[i];
+                }
+            }
+            __syncwarp();
+            mbar_arrive_if(lane == 0, bar(T_EMPTY, ub));
         }
     }
     tc_fence_before();
@@ -515,10 +573,10 @@ struct PrepSlotsArgs {
     float eps;
     int K, rows;              // rows = tokens, or picks (by_pick)
     const int* slot;          // [picks] a pick's place in the sorted list, or -1 (its expert lives elsewhere)
-    int8_t* qi;               // [K / 128][slots][3][128]: the three planes of a slot's 128 values lie together, a chunk's picks in a row
+    uint8_t* planes;          // [K / 256][slots / 8][plane][group][8 slots][64 values] fp16, the 16-byte pieces of a row of 64 swizzled
     int slots;
     float* xscale;            // [slots]
-    float* xsum;              // [slots][K / 64] in units of the slot's scale, which multiplies once at the end of the product
+    float* xsum;              // [slots / 8][K / 64][8] in units of the slot's scale, which multiplies once at the end of the product
 };
 
 // A row is normalised and split once and written to the slots of all its picks (a block per pick normalised every token
@@ -576,26 +634,25 @@ __global__ void __launch_bounds__(256) k_prep_q_slots(const PrepSlotsArgs a) {
     s8 += __shfl_xor_sync(0xffffffffu, s8, 2);
     s8 += __shfl_xor_sync(0xffffffffu, s8, 4);
     if (ok) {
-        uint32_t w[UM_PI][2] = {{0u, 0u}, {0u, 0u}, {0u, 0u}};
+        // q = 2048 h + l in the order of the codes' cells (0, 4, 1, 5, 2, 6, 3, 7); values 1, 3, 5, 7 meet codes in units of 2^-20: times 2^-4
+        uint32_t w[UQ_PL][4] = {{0u, 0u, 0u, 0u}, {0u, 0u, 0u, 0u}};
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            int qv = __float2int_rn(xv[i] * inv * 16384.0f);
-            const int d2 = ((qv + 64) & 127) - 64;
-            qv = (qv - d2) >> 7;
-            const int d1 = ((qv + 64) & 127) - 64;
-            const int d0 = (qv - d1) >> 7;
-            const int sh = 8 * (i >> 1), o = i & 1;               // within 8 values the even ones first, as the codes come out of their nibbles
-            w[0][o] |= (uint32_t)(d0 & 255) << sh; w[1][o] |= (uint32_t)(d1 & 255) << sh; w[2][o] |= (uint32_t)(d2 & 255) << sh;
+            const int qv = __float2int_rn(xv[i] * inv * 16384.0f);
+            const int hi = (qv + 1024) >> 11, lo = qv - (hi << 11);
+            const float f = i & 1 ? 0.0625f : 1.0f;
+            w[0][i & 3] |= (uint32_t)__half_as_ushort(__float2half_rn((float)hi * f)) << (i & 4 ? 16 : 0);
+            w[1][i & 3] |= (uint32_t)__half_as_ushort(__float2half_rn((float)lo * f)) << (i & 4 ? 16 : 0);
         }
         const int np = a.by_pick ? 1 : a.topk;
         for (int r = 0; r < np; r++) {
             const int s = a.slot[row * np + r];
             if (s < 0) continue;
             if (k == 0) a.xscale[s] = mx / 127.0f;
-            if ((lane & 7) == 0) a.xsum[(size_t)s * (a.K >> 6) + (k >> 6)] = mx > 0.f ? s8 / (mx / 127.0f) : 0.f;
+            if ((lane & 7) == 0) a.xsum[((size_t)(s >> 3) * (a.K >> 6) + (k >> 6)) * UQ_G + (s & 7)] = mx > 0.f ? s8 / (mx / 127.0f) : 0.f;
+            uint8_t* dst = a.planes + ((size_t)(k >> 8) * (a.slots / UQ_G) + (s >> 3)) * UQ_GBYTES + ((k >> 6) & 3) * 1024 + (s & 7) * 128 + ((((k >> 3) & 7) ^ (s & 7)) << 4);
 #pragma unroll
-            for (int pl = 0; pl < UM_PI; pl++)
-                *reinterpret_cast<uint2*>(a.qi + ((((size_t)(k >> 7) * a.slots + s) * UM_PI + pl) << 7) + (k & 127)) = make_uint2(w[pl][0], w[pl][1]);
+            for (int pl = 0; pl < UQ_PL; pl++) *reinterpret_cast<uint4*>(dst + pl * UQ_SBO) = make_uint4(w[pl][0], w[pl][1], w[pl][2], w[pl][3]);
         }
     }
     trace_out(a.trace);
