@@ -4,8 +4,8 @@
 //
 //   k_group_picks   counting sort of the step's picks by expert (the host code of
 //                   aegist_rs/src/hybrid.rs:875-900, on the device): per expert the list of its picks in
-//                   pick order, cut into chunks: runs of up to 32 picks (20 for k_umma_q4) go to the "big" table, a rest of
-//                   at most 8 picks (10 for k_umma_q4) to the "small" table (most experts of a step have only a few picks)
+//                   pick order, cut into chunks: runs of up to 32 picks go to the "big" table, a rest of
+//                   at most 8 picks (16 for k_umma_q4) to the "small" table (most experts of a step have only a few picks)
 //   k_mma_q4<NT>    for one chunk (one expert, <= 8 * NT of its picks) and a block of weight rows:
 //                   out = rows x picks, codes widened to fp16 (exact), activations as fp16 hi + lo,
 //                   mma.sync.m16n8k16 into a per-group accumulator that is then scaled:

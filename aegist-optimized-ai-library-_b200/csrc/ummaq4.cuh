@@ -14,29 +14,33 @@
 // 0x000c are the subnormal c 2^-24 and 0x00c0 is c 2^-20, so two masks and a shift turn a nibble pair into operands; the planes of
 // the values that meet the second kind carry 2^-4. Products and the sums of 64 of them are below 2^20 units: exact in the tensor
 // core's fp32 accumulators, whatever its order. One fma joins the planes (rounding once, as a conversion of the whole number would).
-// With int8 planes (three digits, half as many products) the epilogue was what bound the kernel: three columns instead of two per
-// pick, two integer products and a conversion instead of half an fma: 2700 clocks per row block and K step of 20 picks.
+// With int8 planes (three digits, half as many products) the epilogue bound the kernel: three columns per pick instead of two, and two
+// integer products and a conversion instead of half an fma: 2700 clocks per row block and K step of up to 20 picks.
 //
 //   producer warp     per K step (256 codes = 4 groups): one bulk copy with the planes of the chunk's picks (8 KB per eight picks,
-//                     consecutive in memory and laid out as the operand wants them), then per row block the packed codes of 128
-//                     rows (128 bytes each, through a 3-D tensor map [expert][row][byte], 128-byte swizzle). Rings: 2 x 3 x 16 KB of
-//                     codes, 2 x 32 KB of planes
-//   2 table warps     the picks' scales, group sums and output rows of the next unit, and per two K steps the scales and minima of
+//                     consecutive in memory and laid out as the operand wants them; a ring slot holds one, two or four K steps), then
+//                     per row block the packed codes of 128 rows (128 bytes each, through a 3-D tensor map [expert][row][byte],
+//                     128-byte swizzle). Rings: 2 x 2 x 16 KB of codes, 3 x 32 KB of planes (3 and 2 slots: 77 instead of 70 us for
+//                     the gate/up rows of 204 experts, one to eight picks each)
+//   table warp        the picks' scales, group sums and output rows of the next unit, and per two K steps the scales and minima of
 //                     the 256 rows (16 bytes each, cp.async) into a third ring
-//   8 converter warps thread = weight row = TMEM lane: the codes of half a K step -> fp16 straight into tensor memory (tcgen05.st,
-//                     one of four buffers of 64 columns), where tcgen05.mma takes its A operand from. Four warps take the first
-//                     half of every step, four the second: one set alone takes about as long as the copy of the codes
-//   MMA warp          per half step two groups of four tcgen05.mma (kind::f16, M 128, N 32 or 64, K 16) into columns of their own,
-//                     and one commit, which tells the converters that the code buffer is free and the epilogue that the sums are there
-//                     (the barrier cannot run two uses ahead of either: the products of its next use wait for both)
-//   16 epilogue warps thread = weight row = TMEM lane, four warps to a lane quarter, eight picks of both row blocks each: tcgen05.ld of
-//                     two groups, planes joined, times the row's group scale, plus the group minimum times the pick's group sum, group
-//                     after group: a pick's sum has this one order in chunks of every size (k_delta_prompt's note says why that
-//                     matters). Then activation scale and silu(gate) * up, or the picks' output rows
+//   8 converter warps four to a row block; thread = weight row = TMEM lane: the codes of half a K step -> fp16 straight into tensor memory
+//                     (tcgen05.st, one of the row block's two buffers of 64 columns), where tcgen05.mma takes its A operand from
+//   2 MMA warps       one to a row block, so that one's waits lie under the other's products: per half step two groups of four tcgen05.mma
+//                     (kind::f16, M 128, N 16, 32 or 64, K 16) into columns of their own, and commits, which tell the converters that
+//                     the code buffer is free and the epilogue that a buffer of sums is full
+//   8 epilogue warps  four to a row block; thread = weight row = TMEM lane: a buffer is 64 columns, the four groups of up to 8 picks, two of
+//                     up to 16 or one of up to 32: one tcgen05.ld, then four folds of a group of eight picks: planes joined, times the
+//                     row's group scale, plus the group minimum times the picks' group sums. A pick's sum takes its groups in order, in
+//                     chunks of every size (k_delta_prompt's note says why that matters). Then activation scale and
+//                     silu(gate) * up, or the picks' output rows
 //
 // What bounds it, per row block and K step (16 KB of codes, 2 KB of scales: 780 clocks of HBM at the SM's share): sixteen products,
-// which take 44 clocks each for any N up to 80, and commits, which take one product's time; about 850 clocks. So a chunk of 32 picks
-// costs what one pick costs, and eight picks (16 columns: eight of plane h, then eight of plane l) are the step by which lists grow.
+// whose issue takes 44 to 50 clocks each for any N up to 80, whichever warp issues them, and two to four commits, which take one product's time:
+// 800 to 900 clocks; measured 1350 (up to 8 picks, 3.1 TB/s of codes), 1650 (10 picks on average) and 1800 (22). The rest is hand-over: a
+// wait for a phase that is already over takes 55 clocks and more when the SM is busy, a wake-up 114, and there are eleven to fourteen
+// to a row block and K step. So a chunk of 32 picks costs little more than one pick does. us per layer (gate/up + down, 256 experts, 8 picks
+// a token), before and after: 1024 tokens 468 and 260, 333 tokens 215 and 151, 45 tokens 123 and 107, 7 tokens 44 and 46.
 //
 // Every wait is a bounded mbarrier wait; a thread whose wait gave up skips its later waits, the producer stops issuing
 // copies and drains those in flight, and the kernel ends normally with the error word set.
@@ -53,8 +57,9 @@ constexpr int UQ_RAW = UM_M * UQ_KB / 2;         // 16 KB: packed codes of a row
 constexpr int UQ_PL = 2;                         // fp16 planes
 constexpr int UQ_GBYTES = UQ_G * UQ_PL * UQ_KB * 2;      // 8 KB: the planes of eight picks and a K step, [plane][group][pick][64 values]
 constexpr int UQ_SBO = UQ_KB / 64 * 1024;        // bytes between the eight rows of plane h, those of plane l, those of the next eight picks
-constexpr int UQ_PSLOT = UQ_TT / UQ_G * UQ_GBYTES;       // 32 KB
-constexpr int UQ_NW = 3, UQ_NP = 2, UQ_NS = 3;   // ring slots: codes of each row block, planes, row scales
+constexpr int UQ_PSLOT = UQ_TT / UQ_G * UQ_GBYTES;       // 32 KB: a K step of a large chunk, two or four of smaller ones
+__device__ __forceinline__ int uq_ksteps(int picks) { return picks <= UQ_G ? 4 : (picks <= 2 * UQ_G ? 2 : 1); }
+constexpr int UQ_NW = 2, UQ_NP = 3, UQ_NS = 3;   // ring slots: codes of each row block, planes, row scales
 constexpr int UQ_SSLOT = 4 * UM_M * 16;          // 8 KB: [row block][scale | min][128 rows][8 groups] fp16 of two K steps
 constexpr int UQ_MAXG = 32;                      // groups of a row (K <= 2048)
 constexpr int UQ_XS = UQ_TT * UQ_MAXG * 4;       // 4 KB: a unit's group sums, [eight picks][group][pick]
@@ -106,6 +111,15 @@ __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16]
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
                  "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(addr)
                  : "memory");
+}
+// 16 bytes of packed codes -> 16 cells. Eight codes of a word: 0 and 4, 1 and 5, 2 and 6, 3 and 7 to a cell; the planes hold their values in the same order
+__device__ __forceinline__ void uq_cells(const uint4& pk, uint32_t (&o)[16]) {
+    const uint32_t pw[4] = {pk.x, pk.y, pk.z, pk.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        o[4 * i] = pw[i] & 0x000F000Fu; o[4 * i + 1] = pw[i] & 0x00F000F0u;
+        o[4 * i + 2] = (pw[i] >> 8) & 0x000F000Fu; o[4 * i + 3] = (pw[i] >> 8) & 0x00F000F0u;
+    }
 }
 // one arrival when this thread's cp.async copies so far have landed
 __device__ __forceinline__ void mbar_arrive_copies(uint32_t bar) {
@@ -237,16 +251,20 @@ __global__ void __launch_bounds__(UQ_THREADS, 1) k_umma_q4(const __grid_constant
             int e, start, n, r0;
             chunk_of(w, u, e, start, n, r0);
             const uint32_t bytes = (uint32_t)((n + UQ_G - 1) / UQ_G) * UQ_GBYTES;
+            const int ks = uq_ksteps(n);
             for (int kc = 0; kc < nk && !dead; kc++) {
-                wait(bar(P_EMPTY, ps), pph ^ 1, dead);
-                if (dead) break;
-                if (lane == 0) {
-                    mbar_expect_tx(bar(P_FULL, ps), bytes);
-                    bulk_load(ring0 + (uint32_t)(2 * UQ_NW * UQ_RAW + ps * UQ_PSLOT), a.planes + ((size_t)kc * a.slots + start) * (UQ_GBYTES / UQ_G), bytes, bar(P_FULL, ps));
+                if (kc % ks == 0) {
+                    wait(bar(P_EMPTY, ps), pph ^ 1, dead);
+                    if (dead) break;
+                    const int steps = min(ks, nk - kc);
+                    if (lane == 0) mbar_expect_tx(bar(P_FULL, ps), bytes * steps);
+                    __syncwarp();
+                    if (lane < steps)
+                        bulk_load(ring0 + (uint32_t)(2 * UQ_NW * UQ_RAW + ps * UQ_PSLOT) + lane * bytes, a.planes + ((size_t)(kc + lane) * a.slots + start) * (UQ_GBYTES / UQ_G), bytes, bar(P_FULL, ps));
+                    p_armed |= 1u << ps;
+                    p_par = (p_par & ~(1u << ps)) | ((uint32_t)pph << ps);
+                    if (++ps == UQ_NP) { ps = 0; pph ^= 1; }
                 }
-                p_armed |= 1u << ps;
-                p_par = (p_par & ~(1u << ps)) | ((uint32_t)pph << ps);
-                if (++ps == UQ_NP) { ps = 0; pph ^= 1; }
                 for (int rb = 0; rb < 2; rb++) {
                     const int slot = rb * UQ_NW + ws;
                     wait(bar(W_EMPTY, slot), wph ^ 1, dead);
@@ -282,9 +300,12 @@ __global__ void __launch_bounds__(UQ_THREADS, 1) k_umma_q4(const __grid_constant
             const bool big = cn > UQ_SMALL, few = cn <= UQ_FEW;
             bool catch_up = few && !was_few;         // see below
             was_few = few;
+            const int ks = uq_ksteps(cn);
+            const uint32_t bytes = (uint32_t)((cn + UQ_G - 1) / UQ_G) * UQ_GBYTES;
             for (int kc = 0; kc < nk; kc++, kg++) {
-                wait(bar(P_FULL, ps), pph, dead);
-                const uint64_t bd = (umma_desc_sw128(ring0 + (uint32_t)(2 * UQ_NW * UQ_RAW + ps * UQ_PSLOT)) & ~(0x3FFFull << 32)) | ((uint64_t)(UQ_SBO >> 4) << 32);
+                const int kp = kc % ks;
+                if (kp == 0) wait(bar(P_FULL, ps), pph, dead);
+                const uint64_t bd = (umma_desc_sw128(ring0 + (uint32_t)(2 * UQ_NW * UQ_RAW + ps * UQ_PSLOT) + kp * bytes) & ~(0x3FFFull << 32)) | ((uint64_t)(UQ_SBO >> 4) << 32);
 #pragma unroll 1
                 for (int h = 0; h < 2; h++) {
                     const int b = 2 * rb + h;
@@ -327,9 +348,11 @@ __global__ void __launch_bounds__(UQ_THREADS, 1) k_umma_q4(const __grid_constant
                     }
                     __syncwarp();
                 }
-                if (lead) umma_commit(bar(P_EMPTY, ps));
-                __syncwarp();
-                if (++ps == UQ_NP) { ps = 0; pph ^= 1; }
+                if (kp + 1 == ks || kc + 1 == nk) {
+                    if (lead) umma_commit(bar(P_EMPTY, ps));
+                    __syncwarp();
+                    if (++ps == UQ_NP) { ps = 0; pph ^= 1; }
+                }
             }
         }
         if (lead) umma_commit(bar(DRAINED, 0));             // no product may be under way when the block gives its tensor memory back
@@ -389,41 +412,37 @@ __global__ void __launch_bounds__(UQ_THREADS, 1) k_umma_q4(const __grid_constant
         // ---- converters, four warps to a row block: this thread's row of 128 packed bytes -> 2 x 64 cells of two fp16 codes in its TMEM lane ----
         regs_dec<UQ_REGS_LOW>();
         const int q = warp & 3, rb = (warp >> 2) - 1, r = q * 32 + lane;
-        const uint32_t col0 = tmem + ((uint32_t)(q * 32) << 16) + UQ_ACOL + 128u * rb;
+        const uint32_t col0 = held(tmem + ((uint32_t)(q * 32) << 16) + UQ_ACOL + 128u * rb);
+        // the copy's 128-byte swizzle puts 16-byte piece c of row r at c ^ (r & 7), so the same piece of eight neighbouring rows covers all banks
+        const unsigned char* row0 = wring + (size_t)rb * UQ_NW * UQ_RAW + r * 128;
         int st = 0, ph = 0;                          // a ring for each row block: shared, one's converters would pass a barrier by that the other's wait for
         uint32_t kg = 0;
         bool dead = false;
         for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
+#pragma unroll 1
             for (int kc = 0; kc < nk; kc++, kg++) {
                 wait(bar(W_FULL, rb * UQ_NW + st), ph, dead);
-                const unsigned char* row = wring + (size_t)(rb * UQ_NW + st) * UQ_RAW + r * 128;
+                const unsigned char* row = row0 + (size_t)st * UQ_RAW;
 #pragma unroll 1
                 for (int h = 0; h < 2; h++) {
-                    // the copy's 128-byte swizzle puts 16-byte piece c of row r at c ^ (r & 7), so the same piece of eight neighbouring rows covers all banks
                     uint4 pk[4];
 #pragma unroll
                     for (int c = 0; c < 4; c++) pk[c] = *reinterpret_cast<const uint4*>(row + (((4 * h + c) ^ (r & 7)) << 4));
-                    wait(bar(DONE, 2 * rb + h), (kg & 1) ^ 1, dead);                     // the products that read this code buffer are over
+                    wait(bar(DONE, 2 * rb + h), (kg & 1) ^ 1, dead);                 // the products that read this code buffer are over
                     tc_fence_after();
 #pragma unroll
                     for (int c = 0; c < 4; c++) {
-                        // eight codes of a word: 0 and 4, 1 and 5, 2 and 6, 3 and 7 to a cell; the planes hold their values in the same order
-                        const uint32_t pw[4] = {pk[c].x, pk[c].y, pk[c].z, pk[c].w};
                         uint32_t o[16];
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            o[4 * i] = pw[i] & 0x000F000Fu; o[4 * i + 1] = pw[i] & 0x00F000F0u;
-                            o[4 * i + 2] = (pw[i] >> 8) & 0x000F000Fu; o[4 * i + 3] = (pw[i] >> 8) & 0x00F000F0u;
-                        }
+                        uq_cells(pk[c], o);
                         tmem_st16(col0 + 64u * h + 16u * c, o);
                     }
+                    // the stores have taken the codes out of the registers, so their loads have left the ring slot
+                    if (h) mbar_arrive_if(lane == 0, bar(W_EMPTY, rb * UQ_NW + st));
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                     tc_fence_before();
                     __syncwarp();
                     mbar_arrive_if(lane == 0, bar(CONV, 2 * rb + h));
                 }
-                // the stores have taken the codes out of the registers, so their loads have left the ring slot
-                mbar_arrive_if(lane == 0, bar(W_EMPTY, rb * UQ_NW + st));
                 if (++st == UQ_NW) { st = 0; ph ^= 1; }
             }
         }
