@@ -107,7 +107,8 @@ __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
 }
 
 // ---- tcgen05 / TMA wrappers -------------------------------------------------------------------------------------
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+template <typename D, typename B>
+__device__ __forceinline__ void tma_load_2d(D dst, const CUtensorMap* map, int x, int y, B bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
                  "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
                  : "memory");
@@ -303,6 +304,8 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma(const __grid_constant__ 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
+    // shared-memory addresses of the ring and its barriers (held: mbar_wait's note)
+    const uint32_t ring0 = held(smem_u32(ring)), full0 = held(smem_u32(full_bar)), empty0 = held(smem_u32(empty_bar));
     const int NST = um_stages(a.tt), STAGE = um_stage_bytes(a.tt), KC = um_kc(a.tt), CHUNK = um_chunk_bytes(a.tt);
     // token groups of a pass; with a single pass only the groups that hold tokens are counted, so that the work items
     // that exist spread over all blocks
@@ -328,9 +331,13 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma(const __grid_constant__ 
     };
     // A bounded wait. `dead` is the caller's own flag: after one of its waits has given up, a thread skips the rest
     // and runs to the end of its loops; the other roles' waits then give up the same way.
-    auto wait = [&](uint64_t* bar, uint32_t parity, bool& dead) {
+    // Made by whole warps, one lane of which then issues: a single thread's wait took more than twice as long (mbar_wait's note), and the
+    // hand-over of a ring stage is what a K chunk costs.
+    auto wait = [&](auto bar, uint32_t parity, bool& dead) {
         if (dead) return;
-        if (!mbar_wait(bar, parity, a.err, 1 << 21)) dead = true;
+        __syncwarp();
+        dead = !mbar_wait(bar, parity, a.err, 1 << 21);
+        __syncwarp();
     };
     auto locate = [&](int unit, int& s, int& blk) {
         s = 0; blk = unit;
@@ -371,15 +378,15 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma(const __grid_constant__ 
             const Item it = item(w_first);
             for (int k0 = 0; k0 < it.nk && pre < NST; k0 += KC, pre++) {
                 const int nch = min(KC, it.nk - k0);
-                if (lane == 0) mbar_expect_tx(&full_bar[pre], (uint32_t)nch * CHUNK);
+                if (lane == 0) mbar_expect_tx(full0 + 8 * pre, (uint32_t)nch * CHUNK);
                 __syncwarp();
-                if (lane < 5 * nch && which < 2) tma_load_2d(ring + (size_t)pre * STAGE + it.off, it.map, (it.kb + k0 + ck) * UM_BK, it.y, &full_bar[pre]);
+                if (lane < 5 * nch && which < 2) tma_load_2d(ring0 + pre * STAGE + it.off, it.map, (it.kb + k0 + ck) * UM_BK, it.y, full0 + 8 * pre);
             }
             grid_dep_wait();
             if (lane == 0) stamp(1);
             for (int j = 0; j < pre; j++) {
                 const int k0 = j * KC, nch = min(KC, it.nk - k0);
-                if (lane < 5 * nch && which >= 2) tma_load_2d(ring + (size_t)j * STAGE + it.off, it.map, (it.kb + k0 + ck) * UM_BK, it.y, &full_bar[j]);
+                if (lane < 5 * nch && which >= 2) tma_load_2d(ring0 + j * STAGE + it.off, it.map, (it.kb + k0 + ck) * UM_BK, it.y, full0 + 8 * j);
                 armed_mask |= 1u << j;                                  // parity 0: the first use of these stages
             }
             st = pre == NST ? 0 : pre;
@@ -393,13 +400,12 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma(const __grid_constant__ 
             if (!it.ok) continue;
             for (int k0 = (w == w_first ? pre * KC : 0); k0 < it.nk; k0 += KC) {
                 const int nch = min(KC, it.nk - k0);                    // chunks in this stage
-                if (lane == 0) {
-                    wait(&empty_bar[st], ph ^ 1, dead);
-                    if (!dead) mbar_expect_tx(&full_bar[st], (uint32_t)nch * CHUNK);
-                }
-                dead = __shfl_sync(0xffffffffu, (int)dead, 0) != 0;
+                wait(empty0 + 8 * st, ph ^ 1, dead);
+                dead = __any_sync(0xffffffffu, dead);
                 if (dead) break;
-                if (lane < 5 * nch) tma_load_2d(ring + (size_t)st * STAGE + it.off, it.map, (it.kb + k0 + ck) * UM_BK, it.y, &full_bar[st]);
+                if (lane == 0) mbar_expect_tx(full0 + 8 * st, (uint32_t)nch * CHUNK);
+                __syncwarp();
+                if (lane < 5 * nch) tma_load_2d(ring0 + st * STAGE + it.off, it.map, (it.kb + k0 + ck) * UM_BK, it.y, full0 + 8 * st);
                 armed_mask |= 1u << st;
                 armed_par = (armed_par & ~(1u << st)) | ((uint32_t)ph << st);
                 if (++st == NST) { st = 0; ph ^= 1; }
@@ -415,7 +421,8 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma(const __grid_constant__ 
         }
     } else if (warp == 1) {
         // ---- MMA issuer ----
-        if (elect_one()) {
+        {
+            const bool lead = elect_one();
             int st = 0, ph = 0, n = 0;
             bool dead = false;
             // one work item: nk K chunks into accumulator d
@@ -423,12 +430,15 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma(const __grid_constant__ 
                 constexpr bool BF = decltype(bf_)::value != 0;
                 constexpr int TT = decltype(tt_)::value, KCT = um_kc(TT), ST = um_stage_bytes(TT), CH = um_chunk_bytes(TT);
                 for (int k0 = 0; k0 < nk; k0 += KCT) {
-                    wait(&full_bar[st], ph, dead);
+                    wait(full0 + 8 * st, ph, dead);
                     tc_fence_after();
-                    const uint32_t sa = smem_u32(ring) + (uint32_t)st * ST;
-                    um_issue<BF, TT>(d, umma_desc_sw128(sa), umma_desc_sw128(sa + UM_A_BYTES), k0 != 0);
-                    if (KCT == 2 && k0 + 1 < nk) um_issue<BF, TT>(d, umma_desc_sw128(sa + CH), umma_desc_sw128(sa + CH + UM_A_BYTES), true);
-                    umma_commit(&empty_bar[st]);                          // the stage may be refilled once these have read it
+                    const uint32_t sa = ring0 + (uint32_t)st * ST;
+                    if (lead) {
+                        um_issue<BF, TT>(d, umma_desc_sw128(sa), umma_desc_sw128(sa + UM_A_BYTES), k0 != 0);
+                        if (KCT == 2 && k0 + 1 < nk) um_issue<BF, TT>(d, umma_desc_sw128(sa + CH), umma_desc_sw128(sa + CH + UM_A_BYTES), true);
+                        umma_commit(empty0 + 8 * st);                     // the stage may be refilled once these have read it
+                    }
+                    __syncwarp();
                     if (++st == NST) { st = 0; ph ^= 1; }
                 }
             };
@@ -448,10 +458,11 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma(const __grid_constant__ 
                 else if (a.tt == 64) { if (isbf) item(UqInt<1>(), UqInt<64>(), nk, d); else item(UqInt<0>(), UqInt<64>(), nk, d); }
                 else if (a.tt == 32) { if (isbf) item(UqInt<1>(), UqInt<32>(), nk, d); else item(UqInt<0>(), UqInt<32>(), nk, d); }
                 else { if (isbf) item(UqInt<1>(), UqInt<16>(), nk, d); else item(UqInt<0>(), UqInt<16>(), nk, d); }
-                umma_commit(&acc_full[buf]);
+                if (lead) umma_commit(&acc_full[buf]);
+                __syncwarp();
                 n++;
             }
-            stamp(3);
+            if (lead) stamp(3);
         }
         __syncwarp();
     } else if constexpr (SPLIT) {
