@@ -422,14 +422,14 @@ __device__ __forceinline__ bool mbar_try(B bar, uint32_t parity) {
 // the buffer holds, so that the kernel always terminates.
 // The first two tries stand outside the loop: a try blocks for some 5 us when a whole warp makes it, and a warp that is past a loop
 // wakes up 320 clocks after the last arrival, one that is past a plain branch 114 (a phase that is already over: 130 and 55). A wait
-// by one thread of a warp never blocks and polls every 170 clocks, so whole warps wait where it matters. `limit` tries, and about a
-// quarter of a second: a blocking try makes many of them last longer than that.
+// by one thread of a warp never blocks and polls every 170 clocks, so whole warps wait where it matters. The bound counts tries, never
+// time: a block that is switched out (a GPU shared in time slices, a debugger) makes none, and its copies are switched out with it.
+// 2^22 tries are 0.4 s of polls or some 20 s of tries that block.
 template <typename B>
 __device__ __forceinline__ bool mbar_wait(B bar, uint32_t parity, int* err, int limit = 1 << 22) {
     if (mbar_try(bar, parity)) return true;
     if (mbar_try(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (int spin = 2; spin < limit && clock64() - t0 < (1ll << 29); spin++)
+    for (int spin = 2; spin < limit; spin++)
         if (mbar_try(bar, parity)) return true;
     if (err) atomicExch(err, 3);
     return false;

@@ -1,0 +1,56 @@
+"""The bounded waits of the kernels, run on the host: the functions' own source with stand-ins for the instructions they use."""
+import os
+import re
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "aegist-optimized-ai-library-_b200", "csrc")
+
+
+def function(name, file="kernels.cuh"):
+    """The text of one function of a source file, its template line included."""
+    text = open(os.path.join(CSRC, file)).read()
+    m = re.search(r"(?:^template <[^\n]*>\n)?^[^\n/]*\b" + name + r"\(.*?^}\n", text, re.M | re.S)
+    assert m, name
+    return m.group(0)
+
+
+def run(tmp_path, source):
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text("#include <cstdint>\n#include <cstdio>\n#define __device__\n#define __host__\n#define __forceinline__ inline\n" + source)
+    subprocess.run(["g++", "-std=c++20", "-O1", "-pthread", "-o", str(exe), str(src)], check=True)
+    return subprocess.run([str(exe)], check=True, capture_output=True, text=True, timeout=60).stdout.split()
+
+
+@pytest.mark.parametrize("away_after", [1, 2, 3, 10])
+@pytest.mark.parametrize("away", [0, 1 << 31])
+def test_a_wait_outlasts_a_warp_that_was_switched_out(tmp_path, away_after, away):
+    """The warp is off the SM for `away` clocks behind a failed try, and its copy lands a few tries after it is back (it was switched out
+    with it). Only tries that were made count, so the wait succeeds and leaves no error."""
+    assert run(tmp_path, """
+static long long now = 0; static int tries = 0;
+static long long clock64() { return now; }
+static int atomicExch(int* p, int v) { int o = *p; *p = v; return o; }
+template <typename B> static bool mbar_try(B, uint32_t) {
+    ++tries; now += 170;
+    if (tries == %d) now += %dll;
+    return tries == %d + 5;
+}
+""" % (away_after, away, away_after) + function("mbar_wait") + """
+int main() { int err = 0; const bool ok = mbar_wait(0u, 0u, &err); std::printf("%d %d", (int)ok, err); }
+""") == ["1", "0"]
+
+
+@pytest.mark.parametrize("limit", [1, 2, 3, 1000, 1 << 16])
+def test_a_wait_gives_up_after_its_tries(tmp_path, limit):
+    """A phase that never ends: a bounded number of tries (two stand before the loop), then the error word."""
+    ok, err, tries = map(int, run(tmp_path, """
+static long long now = 0; static int tries = 0;
+static long long clock64() { return now; }
+static int atomicExch(int* p, int v) { int o = *p; *p = v; return o; }
+template <typename B> static bool mbar_try(B, uint32_t) { ++tries; now += 170; return false; }
+""" + function("mbar_wait") + """
+int main() { int err = 0; const bool ok = mbar_wait(0u, 0u, &err, %d); std::printf("%%d %%d %%d", (int)ok, err, tries); }
+""" % limit))
+    assert (ok, err) == (0, 3) and tries == max(2, limit)
