@@ -329,16 +329,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma(const __grid_constant__ 
     auto stamp = [&](int i) {
         if (a.trace && blockIdx.x == 0) a.trace[8 + i] = (unsigned long long)clock64();
     };
-    // A bounded wait. `dead` is the caller's own flag: after one of its waits has given up, a thread skips the rest
-    // and runs to the end of its loops; the other roles' waits then give up the same way.
-    // Made by whole warps, one lane of which then issues: a single thread's wait took more than twice as long (mbar_wait's note), and the
-    // hand-over of a ring stage is what a K chunk costs.
-    auto wait = [&](auto bar, uint32_t parity, bool& dead) {
-        if (dead) return;
-        __syncwarp();
-        dead = !mbar_wait(bar, parity, a.err, 1 << 21);
-        __syncwarp();
-    };
+    auto wait = [&](auto bar, uint32_t parity, bool& dead) { warp_wait(bar, parity, a.err, dead); };
     auto locate = [&](int unit, int& s, int& blk) {
         s = 0; blk = unit;
         while (s + 1 < a.nseg && blk >= a.seg[s].units) { blk -= a.seg[s].units; s++; }
@@ -401,7 +392,6 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma(const __grid_constant__ 
             for (int k0 = (w == w_first ? pre * KC : 0); k0 < it.nk; k0 += KC) {
                 const int nch = min(KC, it.nk - k0);                    // chunks in this stage
                 wait(empty0 + 8 * st, ph ^ 1, dead);
-                dead = __any_sync(0xffffffffu, dead);
                 if (dead) break;
                 if (lane == 0) mbar_expect_tx(full0 + 8 * st, (uint32_t)nch * CHUNK);
                 __syncwarp();

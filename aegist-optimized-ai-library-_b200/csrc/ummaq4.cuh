@@ -233,13 +233,7 @@ __global__ void __launch_bounds__(UQ_THREADS, 1) k_umma_q4(const __grid_constant
         e = v.x; start = v.y; n = v.z; r0 = v.w;
     };
     const int rstep = a.pair ? a.up_row0 : UM_M;     // from the first row block to the second
-    // bounded waits of a whole warp; one that gave up skips the rest
-    auto wait = [&](uint32_t at, uint32_t parity, bool& dead) {
-        if (dead) return;
-        __syncwarp();
-        dead = !mbar_wait(at, parity, a.err, 1 << 21);
-        __syncwarp();
-    };
+    auto wait = [&](uint32_t at, uint32_t parity, bool& dead) { warp_wait(at, parity, a.err, dead); };
 
     if (warp < 4) regs_dec<UQ_REGS_LOW>();
     if (warp == 0) {

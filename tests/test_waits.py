@@ -54,3 +54,53 @@ template <typename B> static bool mbar_try(B, uint32_t) { ++tries; now += 170; r
 int main() { int err = 0; const bool ok = mbar_wait(0u, 0u, &err, %d); std::printf("%%d %%d %%d", (int)ok, err, tries); }
 """ % limit))
     assert (ok, err) == (0, 3) and tries == max(2, limit)
+
+
+@pytest.mark.parametrize("never", [0, 1, 1 << 7, 1 << 31, 0x0000FFFF, 0xFFFFFFFE, 0xFFFFFFFF])
+def test_a_warp_that_waits_has_one_verdict(tmp_path, never):
+    """32 threads as a warp: the lanes in `never` never see the phase end, the others at once or, in a second wait, lane i at its i-th try.
+    All lanes must go the same way, or some would meet the others at another barrier or in an instruction of the whole warp; behind a
+    wait that gave up all of them skip the next one."""
+    got = run(tmp_path, """
+#include <atomic>
+#include <barrier>
+#include <thread>
+#include <vector>
+static std::barrier<> meet(32);
+static std::atomic<unsigned> votes, tried;
+static thread_local int lane, tries;
+static int atomicExch(int* p, int v) { return __atomic_exchange_n(p, v, __ATOMIC_SEQ_CST); }
+static void __syncwarp() { meet.arrive_and_wait(); }
+static bool __any_sync(unsigned, bool p) {
+    if (p) votes |= 1u << lane;
+    meet.arrive_and_wait();
+    const bool any = votes != 0;
+    meet.arrive_and_wait();
+    votes = 0;
+    meet.arrive_and_wait();
+    return any;
+}
+static bool __all_sync(unsigned m, bool p) { return !__any_sync(m, !p); }
+template <typename B> static bool mbar_try(B late, uint32_t) {
+    tried++;
+    return late ? ++tries >= lane : !(%uu >> lane & 1);
+}
+""" % never + function("mbar_wait") + function("warp_wait") + """
+int main() {
+    int err = 0;
+    std::atomic<unsigned> gone{0};
+    auto warp = [&](unsigned late) {
+        std::vector<std::thread> t;
+        for (int i = 0; i < 32; i++)
+            t.emplace_back([&, i] { lane = i; bool dead = gone >> i & 1; warp_wait(late, 0u, &err, dead, 64); if (dead) gone |= 1u << i; });
+        for (auto& x : t) x.join();
+    };
+    warp(0);
+    std::printf("%u %d ", gone.load(), err);
+    if (gone != 0 && gone != 0xFFFFFFFFu) return 0;
+    tried = 0;
+    warp(1);
+    std::printf("%u %d", gone.load(), tried > 0);
+}
+""")
+    assert got == (["4294967295", "3", "4294967295", "0"] if never else ["0", "0", "0", "1"])
