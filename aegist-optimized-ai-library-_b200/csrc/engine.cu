@@ -1008,9 +1008,12 @@ static cudaError_t launch_q4(Q4Args q, const ChunkTable& small, const ChunkTable
     return launch_k(k_mma_q4<4>, dim3(row_blocks, gb), dim3(Q4_THREADS), sm4, st, q);
 }
 // The shapes k_umma_q4 takes, and the tensor maps of its two launches (gate/up pairs, down): the pick lists are cut for the kernel
-// that reads them, so whether it can run is known before they are.
+// that reads them, so whether it can run, in this build too (uq_regs_suffice), is known before they are.
 static bool umma_q4_maps(const ExpertArgs& a, const ExpertMmaCtx& m, int P, UmmaQ4Args (&u)[2]) {
     if (!m.sq || !m.experts || q4_slots(P, m.per) > m.slots || m.expert_bytes % 16 != 0 || a.I > 512) return false;       // k_prep_q_slots<2>: 512 values
+    cudaFuncAttributes built;
+    if (cudaFuncGetAttributes(&built, k_umma_q4) != cudaSuccess) { cudaGetLastError(); return false; }
+    if (!uq_regs_suffice(built.numRegs)) return false;
     for (int i = 0; i < 2; i++) {
         const bool pair = i == 0;
         const int K = pair ? a.D : a.I, row_blocks = pair ? a.I : a.D / 2;

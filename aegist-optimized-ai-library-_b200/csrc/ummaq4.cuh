@@ -70,10 +70,14 @@ constexpr int UQ_ACOL = 256;                     // where they start; the accumu
 constexpr int UQ_UNITS = 32;                     // units of a block whose places in the lists are looked up once
 constexpr int UQ_EPI = 8, UQ_CONV = 8;           // epilogue warps, converter warps
 constexpr int UQ_THREADS = (4 + UQ_CONV + UQ_EPI) * 32;  // producer, 2 MMA issuers, tables, converters, epilogue
-// Registers: the block is launched with 96 a thread; producer, issuers, tables and converters (three warpgroups) keep 64 and the epilogue's two
-// get 144: a buffer of 64 columns, the sums of 32 picks and what a fold needs. 3 x 64 + 2 x 144 = 5 x 96
-constexpr int UQ_REGS = 96, UQ_REGS_LOW = 64, UQ_REGS_EPI = 144;
-static_assert(UQ_REGS_LOW * (4 + UQ_CONV) + UQ_REGS_EPI * UQ_EPI <= UQ_REGS * (4 + UQ_CONV + UQ_EPI), "what the epilogue takes has been given back");
+// Registers: producer, issuers, tables and converters (three warpgroups) keep 64 a thread of the 96 that the block is launched with, and the
+// epilogue's two get 144: a buffer of 64 columns, the sums of 32 picks and what a fold needs. 3 x 64 + 2 x 144 = 5 x 96
+constexpr int UQ_REGS_LOW = 64, UQ_REGS_EPI = 144;
+// Whether a launch with `regs` registers a thread, which the compiler decides, has that much to hand over. With fewer the epilogue's
+// setmaxnreg would wait for registers that nobody gives back, the one wait without a bound: such a build must not launch the kernel.
+constexpr bool uq_regs_suffice(int regs) {
+    return regs >= UQ_REGS_LOW && regs <= UQ_REGS_EPI && regs * (4 + UQ_CONV + UQ_EPI) >= UQ_REGS_LOW * (4 + UQ_CONV) + UQ_REGS_EPI * UQ_EPI;
+}
 constexpr size_t UQ_SMEM = (size_t)2 * UQ_NW * UQ_RAW + (size_t)UQ_NP * UQ_PSLOT + (size_t)UQ_NS * UQ_SSLOT + 2 * UQ_XS + UQ_RED + 1024;
 
 struct UmmaQ4Args {

@@ -104,3 +104,27 @@ int main() {
 }
 """)
     assert got == (["4294967295", "3", "4294967295", "0"] if never else ["0", "0", "0", "1"])
+
+
+def test_registers_that_k_umma_q4_hands_over(tmp_path):
+    """setmaxnreg.inc waits without a bound until the block's own pool holds what it asks for. Whatever the compiler made of the kernel, the
+    launch rule says yes only where the epilogue's warpgroups get their registers once the others have given theirs back, and is asked
+    before every launch."""
+    text = open(os.path.join(CSRC, "ummaq4.cuh")).read()
+    lines = [m.group(0) for m in re.finditer(r"^constexpr int UQ_(EPI|THREADS|REGS_LOW)\b.*$", text, re.M)]
+    got = run(tmp_path, "\n".join(lines) + "\n" + function("uq_regs_suffice", "ummaq4.cuh") + """
+int main() {
+    for (int regs = 24; regs * UQ_THREADS <= 65536; regs += 8) {
+        long pool = 0, low = UQ_THREADS / 128 - UQ_EPI / 4;       // warpgroups of 128 threads
+        bool good = regs >= UQ_REGS_LOW && regs <= UQ_REGS_EPI;
+        pool += low * 128 * (regs - UQ_REGS_LOW);
+        for (int g = 0; g < UQ_EPI / 4; g++) { pool -= 128 * (UQ_REGS_EPI - regs); good = good && pool >= 0; }
+        std::printf("%d %d %d ", regs, (int)good, (int)uq_regs_suffice(regs));
+    }
+}
+""")
+    rows = [got[i:i + 3] for i in range(0, len(got), 3)]
+    assert all(good == says for _, good, says in rows)
+    assert {regs: says for regs, _, says in rows}["88"] == "0" and {regs: says for regs, _, says in rows}["96"] == "1"
+    asks = function("umma_q4_maps", "engine.cu")
+    assert "cudaFuncGetAttributes(&built, k_umma_q4)" in asks and "if (!uq_regs_suffice(built.numRegs)) return false;" in asks
