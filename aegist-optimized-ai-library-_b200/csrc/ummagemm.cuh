@@ -286,7 +286,7 @@ __device__ __forceinline__ void um_split_epilogue(const UmmaArgs& a, unsigned ch
 template <bool SPLIT>
 __global__ void __launch_bounds__(UM_THREADS, 1) k_umma(const __grid_constant__ UmmaArgs a) {
     extern __shared__ unsigned char um_raw[];
-    __shared__ __align__(8) uint64_t full_bar[UM_MAX_STAGES], empty_bar[UM_MAX_STAGES], acc_full[2], acc_empty[2];
+    __shared__ __align__(8) uint64_t full_bar[UM_MAX_STAGES], empty_bar[UM_MAX_STAGES], acc_full[2], acc_empty[2], drained;
     __shared__ uint32_t tmem_slot;
     __shared__ float gate_x[SPLIT ? 1 : 2][SPLIT ? 1 : 64][17];      // gate/up pairs: the gate rows' values of 16 tokens, per half of the tokens
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -297,6 +297,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma(const __grid_constant__ 
     if (threadIdx.x == 0) {
         for (int s = 0; s < UM_MAX_STAGES; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
         for (int b = 0; b < 2; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
+        mbar_init(&drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) tmem_alloc(&tmem_slot, UM_TMEM_COLS);
@@ -452,7 +453,10 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma(const __grid_constant__ 
                 __syncwarp();
                 n++;
             }
-            if (lead) stamp(3);
+            // no product may be under way when the block gives its tensor memory back, and an epilogue whose wait gave up waits for none
+            if (lead) { stamp(3); umma_commit(&drained); }
+            __syncwarp();
+            mbar_wait(&drained, 0, a.err, 1 << 21);
         }
         __syncwarp();
     } else if constexpr (SPLIT) {

@@ -128,3 +128,17 @@ int main() {
     assert {regs: says for regs, _, says in rows}["88"] == "0" and {regs: says for regs, _, says in rows}["96"] == "1"
     asks = function("umma_q4_maps", "engine.cu")
     assert "cudaFuncGetAttributes(&built, k_umma_q4)" in asks and "if (!uq_regs_suffice(built.numRegs)) return false;" in asks
+
+
+@pytest.mark.parametrize("file,kernel", [("ummagemm.cuh", "k_umma"), ("ummaq4.cuh", "k_umma_q4")])
+def test_no_product_is_under_way_when_tensor_memory_goes_back(file, kernel):
+    """Products that run on behind a block that has given back its tensor memory, and left, fault. The epilogue has waited for all of them
+    unless one of its waits gave up, so the issuer itself ends with a commit behind its last product and a wait for it."""
+    text = open(os.path.join(CSRC, file)).read()
+    body = text[text.index(" " + kernel + "(const __grid_constant__"):]
+    issuer = re.search(r"// ---- MMA issuer.*?\n    \} else if", body, re.S).group(0)
+    drained, = re.findall(r"umma_commit\(([^;]*drained[^;]*)\);", issuer, re.I)
+    last = max(issuer.rindex("um" + ("_issue<" if kernel == "k_umma" else "ma_commit(bar(P_EMPTY")), issuer.index("umma_commit(" + drained))
+    wait = issuer.index("mbar_wait(" + drained + ", 0, a.err")
+    assert issuer.index("umma_commit(" + drained) == last < wait and "if (dead)" not in issuer[last:wait]
+    assert body.index("mbar_wait(" + drained) < body.index("tmem_dealloc(")
