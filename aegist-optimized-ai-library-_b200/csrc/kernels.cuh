@@ -429,6 +429,7 @@ template <typename B>
 __device__ __forceinline__ bool mbar_wait(B bar, uint32_t parity, int* err, int limit = 1 << 22) {
     if (mbar_try(bar, parity)) return true;
     if (mbar_try(bar, parity)) return true;
+#pragma unroll 1
     for (int spin = 2; spin < limit; spin++)
         if (mbar_try(bar, parity)) return true;
     if (err) atomicExch(err, 3);
@@ -445,6 +446,7 @@ __device__ __forceinline__ void warp_wait(B bar, uint32_t parity, int* err, bool
     if (dead) return;
     if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return;
     if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return;
+#pragma unroll 1
     for (int spin = 2; spin < limit; spin++)
         if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return;
     if (err) atomicExch(err, 3);
