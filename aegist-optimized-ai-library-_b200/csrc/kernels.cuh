@@ -420,11 +420,10 @@ __device__ __forceinline__ bool mbar_try(B bar, uint32_t parity) {
 // Wait for a phase of an mbarrier of this block. The wait is bounded: if the phase has not completed
 // after a very long time (a copy that never lands), *err is set and the caller goes on with whatever
 // the buffer holds, so that the kernel always terminates.
-// The first two tries stand outside the loop: a try blocks for some 5 us when a whole warp makes it, and a warp that is past a loop
-// wakes up 320 clocks after the last arrival, one that is past a plain branch 114 (a phase that is already over: 130 and 55). A wait
-// by one thread of a warp never blocks and polls every 170 clocks, so whole warps wait where it matters. The bound counts tries, never
-// time: a block that is switched out (a GPU shared in time slices, a debugger) makes none, and its copies are switched out with it.
-// 2^22 tries are 0.4 s of polls or some 20 s of tries that block.
+// The first two tries stand outside the loop: a phase that is already over then costs 62 clocks, 111 where the first try is a loop's
+// (a wake-up 116 and 109). A try that fails blocks for 4 us when a whole warp makes it, and a wait by one lane, whose tries do not block,
+// takes 158 clocks and 210: whole warps wait where it matters. The bound counts tries, never time: a block that is switched out (a GPU
+// shared in time slices, a debugger) makes none, and its copies are switched out with it. 2^22 tries take a lane 0.2 s, a warp 17 s.
 template <typename B>
 __device__ __forceinline__ bool mbar_wait(B bar, uint32_t parity, int* err, int limit = 1 << 22) {
     if (mbar_try(bar, parity)) return true;
@@ -439,8 +438,9 @@ __device__ __forceinline__ bool mbar_wait(B bar, uint32_t parity, int* err, int 
 // takes more than twice as long and the hand-over of a ring stage is what a K chunk costs. `dead` is the role's own flag: behind a wait
 // that gave up it skips the rest and runs to the end of its loops; the other roles' waits then give up the same way. Every try has one
 // verdict for all lanes. With one to a lane, lanes that disagreed would part for good: some skip the next barrier, the others meet them in
-// an instruction of the whole warp. It is also faster than mbar_wait between two __syncwarp, as the branches behind a vote need no
-// reconvergence: k_umma_q4 per layer (gate/up + down) 247 -> 235 us at 1024 tokens, 148 -> 130 at 333, 95 -> 87 at 45, 36.5 -> 34.0 at 7.
+// an instruction of the whole warp. In these kernels it is also faster than mbar_wait between two __syncwarp, though not by itself (101 and
+// 128 clocks for a phase that is over and a wake-up, 82 and 124 there; what of it the compiler makes around the branches was not looked
+// into): k_umma_q4 per layer (gate/up + down) 247 -> 235 us at 1024 tokens, 148 -> 130 at 333, 95 -> 87 at 45, 36.5 -> 34.0 at 7.
 template <typename B>
 __device__ __forceinline__ void warp_wait(B bar, uint32_t parity, int* err, bool& dead, int limit = 1 << 21) {
     if (dead) return;

@@ -45,8 +45,9 @@ struct GroupArgs {
     int align;                    // an expert's list starts at a multiple of this
 };
 
-// one block of 1024 threads. An expert's list is in pick order: which chunk a pick falls into decides the order in which
-// k_umma_q4 adds up its groups, so an order left to atomics would change last bits from run to run.
+// one block of 1024 threads. An expert's list is in pick order, so that the same picks lie in the same chunks and places in every run. (A
+// pick's sum has one order wherever it lies. While it followed the size of the chunk, an order left to atomics changed last bits from run
+// to run.)
 __global__ void __launch_bounds__(1024) k_group_picks(const GroupArgs a) {
     __shared__ short s_e[GQ_MAXP];
     __shared__ int s_cnt[256], s_off[256], s_fill[256];

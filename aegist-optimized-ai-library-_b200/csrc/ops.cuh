@@ -23,8 +23,7 @@ static cudaError_t upload(T** dst, const T* src, size_t n) {
 // From this many tokens on the MoE operator's experts run as a grouped GEMM with fp16 hi + lo activations (k_mma_q4), and below
 // it on the small-batch kernels. Not on what the engine runs for 6 or more tokens: k_umma_q4's planes hold
 // an expert activation to 2^-22 of the largest of its pick, and the layer's result was 1.8e-6 to 2.2e-6 off 64-bit arithmetic
-// with them (5.4e-7 to 5.8e-7 as it is). 64 tokens take 459 us a call, 331 with the engine's kernels; 8 tokens 168, 168 on
-// the small-batch kernels.
+// with them (5.4e-7 to 5.8e-7 as it is). 64 tokens take 476 us a call; 8 tokens 168, as on the small-batch kernels.
 constexpr int MOE_GROUP_MIN = 8;
 
 struct b2_moe {

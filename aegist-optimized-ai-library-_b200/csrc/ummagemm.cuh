@@ -6,10 +6,11 @@
 // tensor cores take both operands straight from shared memory and keep the accumulator in tensor memory, so no
 // warp touches a weight byte:
 //
-//   producer warp   one elected lane: TMA tensor copies (cp.async.bulk.tensor, 128-byte swizzle) of a 128-row x 128-byte
-//                   weight box and of the activation planes of the unit's tokens into a 5-stage ring, mbarrier-tracked
-//   MMA warp        one elected lane: tcgen05.mma (M 128, N tokens x planes, K 32 bytes) four times per stage, operands
-//                   described by shared-memory descriptors, accumulators in TMEM; tcgen05.commit releases the stage and,
+//   producer warp   waits for a free stage as a warp, then up to ten lanes issue a TMA tensor copy each (cp.async.bulk.tensor, 128-byte
+//                   swizzle): per K chunk the halves of a 128-row x 128-byte weight box and the unit's three activation planes, into a ring
+//                   of three to five stages, mbarrier-tracked
+//   MMA warp        waits for a full stage as a warp, one elected lane issues tcgen05.mma (M 128, N tokens x planes, K 32 bytes) four times
+//                   per K chunk, operands described by shared-memory descriptors, accumulators in TMEM; tcgen05.commit releases the stage and,
 //                   after the last K chunk, hands the accumulator to the epilogue. Two accumulators alternate, so the
 //                   products of the next unit run under the epilogue of this one.
 //   8 epilogue warps  thread = weight row = TMEM lane (two warps per quarter of the lanes, 16 tokens at a time each): tcgen05.ld, the planes of a token combined, row scale, the
@@ -46,7 +47,7 @@ constexpr int UM_PB = 3;                   // bf16 planes
 constexpr int UM_A_BYTES = UM_M * UM_BK;                     // 16 KB
 constexpr int UM_RING_BYTES = 200 * 1024;
 // A stage holds KC K chunks (each a 128-row x 128-byte weight box + the tokens' planes): the hand-over of a stage between
-// the producer and the MMA lane (two mbarrier operations on either side) costs about 400 cycles whatever it carries, more
+// the producer and the issuer (two mbarrier operations on either side) costs about 400 cycles whatever it carries, more
 // than four products over few tokens take, so units of 32 or 16 tokens move two chunks per stage.
 __host__ __device__ constexpr int um_kc(int tt) { return tt >= 64 ? 1 : 2; }
 __host__ __device__ constexpr int um_chunk_bytes(int tt) { return UM_A_BYTES + tt * UM_PI * UM_BK; }      // 40, 28 or 22 KB
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma(const __grid_constant__ 
     if (warp != 0) grid_dep_wait();
 
     // step-timeline points of block 0 (any thread may stamp): 1 past the dependency wait, 2 the producer has issued its
-    // last copy, 3 the MMA lane has committed its last unit, 4 the epilogue got its first accumulator, 5 the epilogue is done
+    // last copy, 3 the issuing lane has committed its last unit, 4 the epilogue got its first accumulator, 5 the epilogue is done
     auto stamp = [&](int i) {
         if (a.trace && blockIdx.x == 0) a.trace[8 + i] = (unsigned long long)clock64();
     };
@@ -337,7 +338,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_umma(const __grid_constant__ 
     };
 
     if (warp == 0) {
-        // ---- producer: lane 0 waits for the stage and announces the bytes, then lanes 0 .. 5 KC - 1 issue one tensor copy
+        // ---- producer: the warp waits for the stage, lane 0 announces the bytes, then lanes 0 .. 5 KC - 1 issue one tensor copy
         // each: per K chunk the two 64-row halves of the weight box and the three planes ----
         int st = 0, ph = 0;
         bool dead = false;

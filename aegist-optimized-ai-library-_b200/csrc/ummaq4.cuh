@@ -36,22 +36,24 @@
 //                     silu(gate) * up, or the picks' output rows
 //
 // What bounds it, per row block and K step (16 KB of codes, 2 KB of scales: 780 clocks of HBM at the SM's share): sixteen products,
-// whose issue takes 44 to 50 clocks each for any N up to 80, whichever warp issues them, and two to four commits, which take one product's time:
-// 800 to 900 clocks; measured 1350 (up to 8 picks, 3.1 TB/s of codes), 1650 (10 picks on average) and 1800 (22). The rest is hand-over: a
-// wait for a phase that is already over takes 55 clocks and more when the SM is busy, a wake-up 114, and there are eleven to fourteen
-// to a row block and K step. So a chunk of 32 picks costs little more than one pick does. us per layer (gate/up + down, 256 experts, 8 picks
-// a token), before and after: 1024 tokens 468 and 260, 333 tokens 215 and 151, 45 tokens 123 and 107, 7 tokens 44 and 46.
+// whose issue takes 44 to 50 clocks each for any N up to 80, whichever warp issues them, and two and a half to five commits, which take one
+// product's time: 810 to 1050 clocks; measured 1170 (45 tokens: up to 8 picks, 3.6 TB/s of codes), 1450 (333: 10 picks on average) and 1660
+// (1024: 22), gate/up rows, in the block with the most units. The rest is hand-over: a wait for a phase that is already over takes 100 clocks
+// and more when the SM is busy, a wake-up 130, and there are eleven to fourteen to a row block and K step. So a chunk of 32 picks costs
+// little more than one pick does. us per layer (gate/up + down, 256 experts, 8 picks a token) with int8 planes and now: 1024 tokens 468 and
+// 235, 333 tokens 213 and 131, 45 tokens 120 and 87 (prompts); 7 sequences 43 and 34, 64 of Zipf popularity 62 and 45 (in the step's graph).
 //
-// Every wait is a bounded mbarrier wait; a thread whose wait gave up skips its later waits, the producer stops issuing
-// copies and drains those in flight, and the kernel ends normally with the error word set.
+// Every wait is a bounded mbarrier wait of a whole warp; a warp whose wait gave up skips its later waits, the producer stops issuing
+// copies and drains those in flight, and the kernel ends normally with the error word set. setmaxnreg, the one wait that knows no bound, is
+// launched only where it cannot wait for good (uq_regs_suffice).
 #pragma once
 
 namespace b2 {
 
 constexpr int UQ_G = 8;                          // picks whose planes lie together: 16 accumulator columns per group
 constexpr int UQ_FEW = 8;                         // a chunk of at most this many picks has 16 accumulator columns per group, a buffer of 64 for a whole K step;
-constexpr int UQ_SMALL = 16;                     // picks of a small chunk: 32 columns per group, four accumulator buffers of half a K step
-constexpr int UQ_TT = 32;                        // most picks per unit (a chunk of the pick list): 64 columns, two buffers
+constexpr int UQ_SMALL = 16;                     // picks of a small chunk: 32 columns per group, a buffer for half a K step
+constexpr int UQ_TT = 32;                        // most picks per unit (a chunk of the pick list): 64 columns per group, a buffer for each. Two buffers to a row block
 constexpr int UQ_KB = 256;                       // codes per K step: four groups
 constexpr int UQ_RAW = UM_M * UQ_KB / 2;         // 16 KB: packed codes of a row block and K step
 constexpr int UQ_PL = 2;                         // fp16 planes
