@@ -19,11 +19,13 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
 #include "../../include/b200moe.h"
 #include "kernels.cuh"
+#include "step1.cuh"
 #include "nxfile.hpp"
 
 namespace b2 {
@@ -133,7 +135,7 @@ struct b2_engine {
 
     cudaStream_t stream = nullptr;
     cudaGraphExec_t graph = nullptr;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_other = nullptr;
     int launches = 0;
 
     // state
@@ -243,6 +245,24 @@ struct b2_engine {
     int ensure_chunk_bufs(int T);
     int feed_chunk(const uint32_t* ids, int T, bool want_head);
 
+    // The persistent launch that runs a whole step of one sequence (step1.cuh), where the shapes allow it
+    struct Step1 {
+        const void* kernel = nullptr;               // null: steps run as one launch per stage
+        size_t smem = 0;
+        bool off = false;                           // the tapped layers do not allow it
+        int stages = 0;                             // stages of a step: rows of its timeline
+        Step1Layer* layers = nullptr;
+        uint32_t *tiles = nullptr, *epoch = nullptr;
+        S1Copy* copies = nullptr;
+        uint64_t* ll = nullptr;
+        Step1Args args{};
+    } s1;
+    int plan_step1();
+    int upload_step1();
+    int launch_step1(cudaStream_t st);
+    cudaError_t run_graph(cudaGraphExec_t g);
+    bool use_step1() const { return s1.kernel && !s1.off && !profiling; }
+
     // per-kernel timing (b2_profile_step): one event after every launch of an un-graphed step
     bool profiling = false;
     std::vector<cudaEvent_t> prof_ev;
@@ -282,21 +302,25 @@ struct b2_engine {
     std::vector<Piece> state_pieces(int n) const;
 };
 
+static void leave_step1(b2_engine* e);
 b2_engine::~b2_engine() {
     if (t.empty() && !finished) return;   // nothing was ever allocated (e.g. creation was refused)
     cudaSetDevice(device);
+    leave_step1(this);
     if (ep_peer_ready) for (int p = 0; p < ep_world; p++) if (p != ep_rank && ep_peer[p]) cudaIpcCloseMemHandle(ep_peer[p]);
     if (graph) cudaGraphExecDestroy(graph);
     for (auto& kv : t) cudaFree(kv.second.p);
     for (auto& l : layers) { cudaFree((void*)l.eptr); cudaFree(l.router_bias); cudaFree(l.live); }
     void* bufs[] = {conv, state, snap_conv[0], snap_conv[1], snap_state[0], snap_state[1], kpool, vpool, page_table, rope_cos,
                     rope_sin, d_tok, d_next, d_pos, d_err, d_hist, d_counter, d_acounter, x, big, zbuf, kraw, vraw, beta, gdec, obuf, att,
-                    rlogits, sh_act, sgate, act, logits, top_idx, top_w, part_val, part_idx, attn_part, tap_buf, ypart, d_dcounter, rec_local, ep_block, d_ep_seq, d_ep_rows, xh, g_list, g_slot, g_chunk, acth, xsum_tok, xsum_act, sq, sq_scale, sq_sum, d_trace, (void*)top_ptr, actq, asc, asum, uq_i, uq_b, uq_scale, d_counts, csel, cselw, cscore, core_y};
+                    rlogits, sh_act, sgate, act, logits, top_idx, top_w, part_val, part_idx, attn_part, tap_buf, ypart, d_dcounter, rec_local, ep_block, d_ep_seq, d_ep_rows, xh, g_list, g_slot, g_chunk, acth, xsum_tok, xsum_act, sq, sq_scale, sq_sum, d_trace, (void*)top_ptr, actq, asc, asum, uq_i, uq_b, uq_scale, d_counts, csel, cselw, cscore, core_y,
+                    s1.layers, s1.tiles, s1.copies, s1.epoch, s1.ll};
     for (void* p : bufs) cudaFree(p);
     free_chunk_bufs();
     if (h_pin) cudaFreeHost(h_pin);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
+    if (ev_other) cudaEventDestroy(ev_other);
     for (cudaEvent_t e : prof_ev) cudaEventDestroy(e);
     if (comm && p_ncclCommDestroy) p_ncclCommDestroy(comm);
     if (stream) cudaStreamDestroy(stream);
@@ -607,6 +631,7 @@ int b2_engine::finish() {
     CU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CU(cudaEventCreate(&ev0));
     CU(cudaEventCreate(&ev1));
+    CU(cudaEventCreateWithFlags(&ev_other, cudaEventDisableTiming));
     CU(cudaDeviceSynchronize());
     finished = true;
     char buf[512];
@@ -616,6 +641,7 @@ int b2_engine::finish() {
              kv_f32 ? "fp32" : "bf16", kv_bytes / 1e9);
     desc = buf;
     if (ep_world > 1) return 0;   // the step graph holds NCCL calls: it is built by b2_ep_init
+    if (plan_step1()) return 1;
     return build_graph();
 }
 
@@ -1209,6 +1235,10 @@ static cudaError_t launch_moe1(const Cfg& c, const float* rlogits, const float* 
 // every matrix product; conv, delta rule and attention walk them in order; the head runs for the last token only,
 // and only when chunk_head is set).
 int b2_engine::enqueue_step(cudaStream_t st, bool count, int chunk_T, bool chunk_head) {
+    if (chunk_T == 0 && use_step1()) {
+        if (count) launches = s1.stages;
+        return launch_step1(st);
+    }
     int n = 0;
     const int launches0 = g_launch_count;
     const bool chunk = chunk_T > 0;
@@ -1542,9 +1572,269 @@ int b2_engine::feed_chunk(const uint32_t* ids, int T, bool want_head) {
     return 0;
 }
 
+// ---- the persistent launch of a step of one sequence (step1.cuh) ---------------------------------------------------
+struct Step1Shape { int sd, so, dk, hd, gh; const void* kernel; int smem_rest; };
+#define S1_SHAPE(sd, so, dk, hd, gh) {sd, so, dk, hd, gh, (const void*)k_step1<sd, so, dk, hd, gh>, Step1Smem<sd, so, hd, gh>::TOTAL}
+// widths the kernel is built for: d_model / 16, the mixers' output width / 16, key width of the delta rule, head width, expert
+// hidden / 128
+static const Step1Shape STEP1_SHAPES[] = {S1_SHAPE(32, 32, 64, 128, 1), S1_SHAPE(64, 128, 128, 128, 2), S1_SHAPE(128, 128, 128, 128, 4), S1_SHAPE(128, 256, 128, 256, 4)};
+
+// Rows of several matrices dealt out to G blocks in one go: block b owns the rows that start in its share of all bytes, in order, cut into
+// tiles of at most seg.maxn rows. False if a block gets more tiles than it has room for.
+struct Step1Seg { int rows, unit, maxn; };
+static bool deal_tiles(const std::vector<Step1Seg>& segs, int G, int kind, std::vector<uint32_t>& tiles) {
+    long total = 0, at = 0;
+    for (const Step1Seg& s : segs) total += (long)s.rows * s.unit;
+    std::vector<int> n(G, 0), last(G, -1);
+    for (size_t si = 0; si < segs.size(); si++)
+        for (int r = 0; r < segs[si].rows; r++, at += segs[si].unit) {
+            int b = (int)(at * G / total);
+            while (b + 1 < G && (long)(b + 1) * total / G <= at) b++;
+            while (b > 0 && (long)b * total / G > at) b--;
+            uint32_t* t = &tiles[(size_t)b * S1_TILES + s1_at(kind)];
+            if (n[b] > 0 && last[b] == (int)si && (int)((t[n[b] - 1] >> 24) & 31) < segs[si].maxn) { t[n[b] - 1] += 1u << 24; continue; }
+            if (n[b] == s1_cap(kind)) return false;
+            t[n[b]++] = s1_tile((int)si, 1, r);
+            last[b] = (int)si;
+        }
+    return true;
+}
+
+// The same where a few rows (`heavy`) take long to multiply: whole tiles of them go to blocks far apart, and the other rows fill the blocks up
+// to an even height.
+static bool deal_spread(const std::vector<Step1Seg>& heavy, const std::vector<Step1Seg>& rest, int G, int kind, std::vector<uint32_t>& tiles) {
+    std::vector<int> n(G, 0);
+    std::vector<long> used(G, 0);
+    int nt = 0, at = 0;
+    for (const Step1Seg& s : heavy) nt += (s.rows + s.maxn - 1) / s.maxn;
+    for (size_t si = 0; si < heavy.size(); si++)
+        for (int r = 0; r < heavy[si].rows; r += heavy[si].maxn, at++) {
+            const int b = (int)((long)at * G / nt), m = std::min(heavy[si].maxn, heavy[si].rows - r);
+            if (n[b] == s1_cap(kind)) return false;
+            tiles[(size_t)b * S1_TILES + s1_at(kind) + n[b]++] = s1_tile((int)si, m, r);
+            used[b] += (long)m * heavy[si].unit;
+        }
+    long rows = 0;
+    for (const Step1Seg& s : rest) rows += s.rows;
+    long height = 0, room = 0;
+    while (room < rows) {
+        height++;
+        room = 0;
+        for (int b = 0; b < G; b++) room += std::max(0L, height - used[b]);
+    }
+    int b = 0;
+    for (size_t si = 0; si < rest.size(); si++)
+        for (int r = 0; r < rest[si].rows;) {
+            while (b < G && used[b] >= height) b++;
+            if (b == G || n[b] == s1_cap(kind)) return false;
+            const int m = (int)std::min<long>({(long)rest[si].maxn, (long)rest[si].rows - r, height - used[b]});
+            tiles[(size_t)b * S1_TILES + s1_at(kind) + n[b]++] = s1_tile((int)(heavy.size() + si), m, r);
+            used[b] += m;
+            r += m;
+        }
+    return true;
+}
+
+// Decides whether steps of this engine run as one persistent launch, and lays out what that needs. Not an error if they do not.
+int b2_engine::plan_step1() {
+    const int G = nsm;
+    if (B != 1 || ep_world != 1 || live_cores > 0 || getenv("B2_NO_STEP1")) return 0;
+    const int hr = c.RD / 2;
+    const bool rope_ok = c.RD > 0 && c.RD <= c.HD && hr % std::max(1, c.HD / 32) == 0;
+    if (c.G != 64 || c.CK != 4 || c.TOPK > 8 || c.E > 256 || c.E % 8 || c.SH % 32 || c.SH > 512 || c.I % 128 || !rope_ok || c.H % c.KV || c.H / c.KV > 8 || c.KV > G ||
+        c.HV % std::max(c.HK, 1) || (c.DV != 64 && c.DV != 128) || c.H * c.HD != c.VD() || c.D < G || (c.D + G - 1) / G > 16 || c.TOPK * c.I < G ||
+        (c.TOPK * c.I + G - 1) / G > 32 || (c.n1 + c.n2) % 2 || c.V < G || c.V >= 1 << 24 ||
+        c.V % 8 || c.C() % 8 || c.VD() % 8 || c.HV % 8 || (c.KV * c.HD) % 8 || c.SH % 8 || c.D % 8) return 0;       // (the last: 16-byte pieces of their scales)
+    const Step1Shape* sh = nullptr;
+    for (const Step1Shape& s : STEP1_SHAPES)
+        if (s.sd * 16 == c.D && s.so * 16 == c.VD() && s.dk == c.DK && s.hd == c.HD && s.gh * 128 == c.I) sh = &s;
+    if (!sh) return 0;
+    const int ns = G / c.KV, chunk = std::max(16, (cap + ns - 1) / ns);
+    if ((chunk + KV_PAGE - 1) / KV_PAGE + 1 > S1_PAGES) return 0;
+    // tiles: as many rows as make the longest share of the DeltaNet in-projections (the largest stage) a whole number of them
+    const int VD = c.VD(), KO = VD, rd = (c.D + G - 1) / G, gp = (c.TOPK * c.I + G - 1) / G;
+    const long u = ((long)c.C() + VD + 4L * c.HV + G - 1) / G;
+    const int r = (int)((u + (u + 15) / 16 - 1) / ((u + 15) / 16));
+    const int n8 = r, nb = std::max(1, std::min(8, r / 2)), no = std::max(1, std::min(8, (rd + 1) / 2)), np = std::max(1, std::min(8, r / 2 / 2 * 2));
+    const int h8 = s1_half_at(n8, c.D), hb = s1_half_at(nb, 2 * c.D), ho = s1_half_at(no, KO), hp = s1_half_at(np, c.D), hs = s1_half_at(rd, c.SH);
+    const int stage = (std::max({h8 + n8 / 2 * c.D, hb + nb / 2 * 2 * c.D, ho + no / 2 * KO, 3 * hp + np / 2 * c.D, hs + rd / 2 * c.SH,
+                                 gp * (c.D / 2) + 64, c.TOPK * s1_dn_stride(rd, c.I / 2), 16 * c.HD * (kv_f32 ? 4 : 2), 4 * s1_gsc_stride(c.D) + 2 * c.TOPK * s1_dsc_stride(c.I)}) + 15) / 16 * 16;
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, sh->kernel) != cudaSuccess) { cudaGetLastError(); return 0; }
+    if (!s1_regs_suffice(fa.numRegs)) return 0;
+    const long room = 227 * 1024 - (long)fa.sharedSizeBytes - sh->smem_rest;
+    const int nst = (int)std::min<long>(S1_MAXST, room / (stage + S1_OPS));
+    if (nst < 5) return 0;         // the attention looks at two tiles of keys while their values are on their way, the experts at three of four
+    std::vector<uint32_t> tiles((size_t)G * S1_TILES, S1_NONE);
+    if (!deal_spread({{c.HV, 2, nb}, {c.HV, 2, nb}}, {{c.C(), 1, n8}, {VD, 1, n8}}, G, S1_IN_DELTA, tiles) ||
+        !deal_tiles({{2 * c.H * c.HD, 1, n8}, {c.KV * c.HD, 1, n8}, {c.KV * c.HD, 1, n8}}, G, S1_IN_ATTN, tiles) ||
+        !deal_tiles({{c.D, 1, no}}, G, S1_OUT, tiles) ||
+        !deal_tiles({{c.E, 1, nb}, {c.n1, 1, nb}, {c.n2, 1, nb}, {1, 1, nb}, {c.SH, 1, np}}, G, S1_MOE, tiles) ||
+        !deal_tiles({{c.D, 1, 16}}, G, S1_SHD, tiles)) return 0;
+    // every block has its rows of the residual stream where the kernel expects them
+    for (int b = 0; b < G; b++) {
+        const uint32_t t = tiles[(size_t)b * S1_TILES + s1_at(S1_SHD)];
+        const int r0 = (int)((long)b * c.D / G), r1 = (int)((long)(b + 1) * c.D / G);
+        if (t != s1_tile(0, r1 - r0, r0) || (int)(tiles[(size_t)b * S1_TILES + s1_at(S1_OUT)] & 0xffffff) != r0) return 0;
+    }
+    // the copies that fetch a tile: its two halves (four of a tile of gate-up pairs) and what the epilogue needs of its rows
+    std::vector<S1Copy> copies((size_t)G * S1_TILES * S1_COPIES, S1Copy{0, 0});
+    bool fits = true;
+    for (int b = 0; b < G; b++)
+        for (int kind = 0; kind < S1_KINDS; kind++)
+            for (int i = 0; i < s1_cap(kind); i++) {
+                const size_t ti = (size_t)b * S1_TILES + s1_at(kind) + i;
+                if (tiles[ti] == S1_NONE) break;
+                const int seg = tiles[ti] >> 29, n = (tiles[ti] >> 24) & 31, row0 = tiles[ti] & 0xffffff, h = (n + 1) / 2;
+                S1Copy* to = &copies[ti * S1_COPIES];
+                auto put = [&](int ptr, size_t from, size_t bytes, int at) {
+                    if (bytes == 0) return;
+                    if (from % 16 || bytes % 16 || at % 16 || bytes / 16 >= 4096 || at / 16 >= 2048 || from / 16 > 0xffffffffull || to == &copies[(ti + 1) * S1_COPIES]) { fits = false; return; }
+                    *to++ = S1Copy{(uint32_t)ptr | (uint32_t)(at / 16) << 5 | (uint32_t)(bytes / 16) << 16, (uint32_t)(from / 16)};
+                };
+                const bool pair = kind == S1_MOE && seg == 4;
+                const size_t rb = s1_is_bf(kind, seg) ? 2 * c.D : (kind == S1_OUT ? KO : (kind == S1_SHD ? c.SH : c.D));
+                const int half = s1_is_bf(kind, seg) ? hb : (kind == S1_OUT ? ho : (kind == S1_SHD ? hs : (pair ? hp : h8)));
+                const int ptr = kind <= S1_IN_ATTN ? seg : (kind == S1_OUT ? W_OUT : (kind == S1_MOE ? W_ROUTER + seg : W_SHD));
+                for (int u = 0; u < (pair ? 2 : 1); u++) {
+                    put(u ? (int)W_UP : ptr, row0 * rb, h * rb, u * 2 * hp);
+                    put(u ? (int)W_UP : ptr, (row0 + h) * rb, (n - h) * rb, u * 2 * hp + half);
+                }
+                auto op = [&](int ptr, size_t size, int at) {
+                    const size_t from = row0 * size / 16 * 16, end = ((row0 + n) * size + 15) / 16 * 16;
+                    put(ptr, from, end - from, stage + at);
+                };
+                if (kind == S1_IN_DELTA && seg == 1) { op(Q_A_LOG, 2, 0); op(Q_DT, 2, 64); }
+                if (kind == S1_IN_DELTA && seg >= 2) op(S_IN + seg - 2, 2, 0);
+                if (kind == S1_IN_DELTA && seg == 2) { op(Q_CONV_W, 8, 128); op(Q_CONV_STATE, 12, 272); }
+                if (kind == S1_IN_ATTN) op(S_IN + seg, 2, 0);
+                if (kind == S1_OUT) op(S_OUT, 2, 0);
+                if (kind == S1_SHD) op(S_SHD, 2, 0);
+                if (kind == S1_MOE && seg == 0) op(Q_BIAS, 4, 64);
+                if (pair) { op(S_GATE, 2, 0); op(S_UP, 2, 64); }
+            }
+    if (!fits) return 0;
+    const size_t smem = (size_t)nst * (stage + S1_OPS) + sh->smem_rest;
+    int per_sm = 0;
+    if (cudaFuncSetAttribute(sh->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sh->kernel, S1_THREADS, smem) != cudaSuccess || per_sm < 1) { cudaGetLastError(); return 0; }
+    Step1Args& a = s1.args;
+    uint32_t at = 0;
+    auto part = [&](uint32_t n) { const uint32_t o = at; at += (n + 15) / 16 * 16; return o; };
+    a.o_xa = part(c.D); a.o_xb = part(c.D); a.o_q = part(std::max(c.C(), (2 * c.H + 2 * c.KV) * c.HD)); a.o_z = part(VD); a.o_bg = part(2 * c.HV);
+    a.o_og = part(KO); a.o_rl = part(c.E); a.o_sa = part(c.SH); a.o_sg = part(1); a.o_act = part(c.TOPK * c.I);
+    a.ll_set = at;
+    at *= 2;
+    a.o_ap = part(c.KV * ns * 8 * (c.HD + 2)); a.cs_words = (c.n1 + c.n2 + 15) / 16 * 16; a.o_cs = part(c.L * a.cs_words);
+    CU(dalloc(&s1.ll, at));
+    CU(dalloc(&s1.tiles, tiles.size(), false));
+    CU(cudaMemcpy(s1.tiles, tiles.data(), tiles.size() * 4, cudaMemcpyHostToDevice));
+    CU(dalloc(&s1.copies, copies.size(), false));
+    CU(cudaMemcpy(s1.copies, copies.data(), copies.size() * sizeof(S1Copy), cudaMemcpyHostToDevice));
+    CU(dalloc(&s1.epoch, 1));
+    CU(dalloc(&s1.layers, c.L, false));
+    if (G > head_grid) {                       // the arg-max' scratch: one place per block
+        cudaFree(part_val); cudaFree(part_idx);
+        part_val = nullptr; part_idx = nullptr;
+        CU(dalloc(&part_val, G)); CU(dalloc(&part_idx, G));
+    }
+    a.layers = s1.layers; a.tiles = s1.tiles; a.embed = embed; a.norm = norm; a.head_w = lm_head.w; a.head_s = lm_head.s; a.logits = logits; a.x = x; a.ll = s1.ll;
+    a.epoch = s1.epoch; a.rope_cos = rope_cos; a.rope_sin = rope_sin; a.page_table = page_table; a.scale = 1.0f / std::sqrt((float)c.HD); a.eps = c.eps;
+    a.L = c.L; a.V = c.V; a.E = c.E; a.topk = c.TOPK; a.I = c.I; a.SH = c.SH; a.HK = c.HK; a.HV = c.HV; a.DV = c.DV; a.H = c.H; a.KV = c.KV; a.RD = c.RD; a.C = c.C();
+    a.n1 = c.n1; a.n2 = c.n2; a.cores_k = c.cores_active; a.kv_f32 = kv_f32; a.half_i8 = h8; a.half_bf = hb; a.half_out = ho; a.half_pair = hp; a.half_shd = hs; a.copies = s1.copies; a.kv_tile = std::min(64, stage / (c.HD * (kv_f32 ? 4 : 2))); a.head_rows = n8; a.nst = nst; a.stage_bytes = stage + S1_OPS;
+    a.expert_bytes = c.expert_bytes(); a.off_gu_s = c.off_gu_s(); a.off_gu_m = c.off_gu_m(); a.off_dn_q = c.off_dn_q(); a.off_dn_s = c.off_dn_s(); a.off_dn_m = c.off_dn_m();
+    a.cscore = cscore; a.csel = csel; a.cselw = cselw; a.part_val = part_val; a.part_idx = part_idx; a.next_tok = d_next; a.pos = d_pos; a.tok = d_tok;
+    a.hist = TokHist{d_hist, cap, 1}; a.counter = d_counter; a.err = d_err;
+    s1.smem = smem;
+    s1.stages = 1;
+    for (const LayerW& l : layers) s1.stages += l.attn ? 7 : 6;
+    if (s1.stages > TRACE_MAX_LAUNCHES) return 0;
+    s1.kernel = sh->kernel;
+    return 0;
+}
+
+// The table of the layers' pointers; again whenever the tapped layers change. A layer tapped twice has one place only: launches per stage then.
+int b2_engine::upload_step1() {
+    if (!s1.layers) return 0;
+    s1.off = false;
+    std::vector<Step1Layer> tab(c.L);
+    const size_t kv_layer = (size_t)pages_per_seq * c.KV * KV_PAGE * c.HD * (kv_f32 ? 4 : 2);
+    for (int i = 0; i < c.L; i++) {
+        const LayerW& l = layers[i];
+        Step1Layer& t = tab[i];
+        t = Step1Layer{};
+        auto put = [&](int wi, int si, const QWd& q) { t.w[wi] = q.w; if (si >= 0) t.s[si] = q.s; };
+        if (l.attn) {
+            put(0, 0, l.q); put(1, 1, l.k); put(2, 2, l.v); put(4, 3, l.o);
+            t.n_a = l.q_norm; t.n_b = l.k_norm;
+            t.kpool = (char*)kpool + kv_layer * l.slot; t.vpool = (char*)vpool + kv_layer * l.slot;
+        } else {
+            t.w[0] = l.in_b; t.w[1] = l.in_a; put(2, 0, l.in_qkv); put(3, 1, l.in_z); put(4, 3, l.out);
+            t.n_a = l.gnorm; t.conv_w = l.conv; t.a_log = l.a_log; t.dt_bias = l.dt_bias;
+            t.conv_state = conv + (size_t)l.slot * c.C() * 3; t.state = state + (size_t)l.slot * c.HV * c.DK * c.DV;
+        }
+        t.w[5] = l.router; t.w[6] = l.key1 ? l.key1 : l.router; t.w[7] = l.key2 ? l.key2 : l.router; t.w[8] = l.sh_gw;      // without a core engine the key rows are not looked at
+        put(9, 4, l.sh_gate); put(10, 5, l.sh_up); put(11, 6, l.sh_down);
+        t.norm1 = l.norm1; t.norm2 = l.norm2; t.bias = l.router_bias; t.experts = l.experts;
+        t.counts = l.key1 ? d_counts + (size_t)i * c.n1 * c.n2 : nullptr;
+        t.top_idx = top_idx + (size_t)i * c.TOPK; t.top_w = top_w + (size_t)i * c.TOPK; t.attn = l.attn;
+        int taps = 0;
+        for (size_t j = 0; j < tap_layers.size(); j++)
+            if (tap_layers[j] == i) { t.tap = tap_buf + j * (size_t)c.D; taps++; }
+        if (taps > 1) s1.off = true;
+    }
+    CU(cudaMemcpy(s1.layers, tab.data(), tab.size() * sizeof(Step1Layer), cudaMemcpyHostToDevice));
+    return 0;
+}
+
+int b2_engine::launch_step1(cudaStream_t st) {
+    Step1Args a = s1.args;
+    a.trace = g_trace_base;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nsm);
+    cfg.blockDim = dim3(S1_THREADS);
+    cfg.dynamicSmemBytes = s1.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;       // its blocks wait on one another
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    void* p[] = {&a};
+    g_launch_count++;
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, s1.kernel, p);
+    if (e != cudaSuccess) return fail("step launch: %s", cudaGetErrorString(e));
+    return 0;
+}
+
+// Persistent launches of two engines of a process must not hold half of a GPU's SMs each and wait for the other half: an engine that
+// follows another one on a device waits for what that one has enqueued so far. Nothing is added while one engine is used.
+static std::mutex g_step1_mutex;
+static std::map<int, b2_engine*> g_step1_last;          // device -> the engine whose step was launched last
+cudaError_t b2_engine::run_graph(cudaGraphExec_t g) {
+    if (!use_step1()) return cudaGraphLaunch(g, stream);
+    std::lock_guard<std::mutex> lock(g_step1_mutex);
+    b2_engine*& last = g_step1_last[device];
+    if (last && last != this) {
+        cudaError_t e = cudaEventRecord(ev_other, last->stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, ev_other, 0);
+        if (e != cudaSuccess) return e;
+    }
+    last = this;
+    return cudaGraphLaunch(g, stream);
+}
+static void leave_step1(b2_engine* e) {
+    if (!e->s1.layers) return;
+    std::lock_guard<std::mutex> lock(g_step1_mutex);
+    if (e->stream) cudaStreamSynchronize(e->stream);
+    auto it = g_step1_last.find(e->device);
+    if (it != g_step1_last.end() && it->second == e) g_step1_last.erase(it);
+}
+
 int b2_engine::build_graph() {
     CU(cudaSetDevice(device));
     if (graph) { cudaGraphExecDestroy(graph); graph = nullptr; }
+    if (upload_step1()) return 1;
     cudaGraph_t g;
     CU(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     int rc = enqueue_step(stream, true);
@@ -1577,7 +1867,7 @@ int b2_engine::check_device_error() {
 }
 
 int b2_engine::run_steps(int n) {
-    for (int i = 0; i < n; i++) CU(cudaGraphLaunch(graph, stream));
+    for (int i = 0; i < n; i++) CU(run_graph(graph));
     if (ep_world > 1) ep_steps += n;
     length += n;
     hits += (uint64_t)n * B * c.TOPK * c.L;
@@ -2150,6 +2440,7 @@ int b2_set_router_bias(b2_engine* e, int layer, const float* bias) {
 }
 
 int b2_launches_per_step(const b2_engine* e) { return e ? e->launches : 0; }
+int b2_kernels_per_step(const b2_engine* e) { return !e ? 0 : (e->use_step1() ? 1 : e->launches); }
 long b2_debug_umma_launches(void) { return g_umma_launches; }
 void b2_debug_refuse_tensor_maps(int on) { g_refuse_maps = on != 0; }
 
@@ -2202,14 +2493,14 @@ int b2_debug_trace_step(b2_engine* e, unsigned long long* out, int cap_launches,
     g_trace_first = g_launch_count;
     cudaError_t ce = cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal);
     int rc = ce == cudaSuccess ? e->enqueue_step(e->stream, false) : 1;
-    const int n = g_launch_count - g_trace_first;
+    const int n = e->use_step1() ? e->s1.stages : g_launch_count - g_trace_first;
     g_trace_base = nullptr;
     cudaError_t ce2 = cudaStreamEndCapture(e->stream, &g);
     if (rc || ce != cudaSuccess || ce2 != cudaSuccess) return e->fail("trace step: capture failed");
     ce = cudaGraphInstantiate(&ge, g, 0);
     cudaGraphDestroy(g);
     if (ce != cudaSuccess) return e->fail("trace step: %s", cudaGetErrorString(ce));
-    ce = cudaGraphLaunch(ge, e->stream);
+    ce = e->run_graph(ge);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
     cudaGraphExecDestroy(ge);
     if (ce != cudaSuccess) return e->fail("trace step: %s", cudaGetErrorString(ce));

@@ -415,7 +415,7 @@ __global__ void __maxnreg__(56) k_moe_gu1(const Gu1Args a) {
     {
         float w0, w1;
         plane_weights(tid, s_scale, w0, w1);
-        float vg = accg[0] * w0 + accg[1] * w1, vu = accu[0] * w0 + accu[1] * w1;
+        float vg = fmaf(accg[0], w0, __fmul_rn(accg[1], w1)), vu = fmaf(accu[0], w0, __fmul_rn(accu[1], w1));      // (spelt out: k_step1 has to round alike)
         vg += __shfl_xor_sync(0xffffffffu, vg, 1); vu += __shfl_xor_sync(0xffffffffu, vu, 1);
         if (tid == 0) { s_part[ke][rb][gid][0] = vg + mng; s_part[ke][rb][gid][1] = vu + mnu; }
     }
@@ -566,10 +566,10 @@ __global__ void __launch_bounds__(M1_DOWN_WARPS * 32) k_moe_down1(const Down1Arg
                 imma16832(t1, a01 & 0x0F0F0F0Fu, a11 & 0x0F0F0F0Fu, (a01 >> 4) & 0x0F0F0F0Fu, (a11 >> 4) & 0x0F0F0F0Fu, xb1.x, xb1.y);
                 const float c0 = s_as[2 * g], c1 = s_as[2 * g + 1];           // scales of the two 32-value groups
                 const float xs = s_as[2 * gh + 2 * g] + s_as[2 * gh + 2 * g + 1];
-                const float v0 = c0 * (small_int_to_float(t0[0]) * pw0 + small_int_to_float(t0[1]) * pw1) +
-                                 c1 * (small_int_to_float(t1[0]) * pw0 + small_int_to_float(t1[1]) * pw1);
-                const float v1 = c0 * (small_int_to_float(t0[2]) * pw0 + small_int_to_float(t0[3]) * pw1) +
-                                 c1 * (small_int_to_float(t1[2]) * pw0 + small_int_to_float(t1[3]) * pw1);
+                const float v0 = fmaf(c0, fmaf(small_int_to_float(t0[0]), pw0, __fmul_rn(small_int_to_float(t0[1]), pw1)),
+                                      __fmul_rn(c1, fmaf(small_int_to_float(t1[0]), pw0, __fmul_rn(small_int_to_float(t1[1]), pw1))));
+                const float v1 = fmaf(c0, fmaf(small_int_to_float(t0[2]), pw0, __fmul_rn(small_int_to_float(t0[3]), pw1)),
+                                      __fmul_rn(c1, fmaf(small_int_to_float(t1[2]), pw0, __fmul_rn(small_int_to_float(t1[3]), pw1))));
                 y0 = fmaf(h2f(s0[g]), v0, y0);
                 y1 = fmaf(h2f(s1[g]), v1, y1);
                 m0 = fmaf(h2f(s0[ngroup + g]), xs, m0);
@@ -628,8 +628,8 @@ __global__ void __launch_bounds__(M1_DOWN_WARPS * 32) k_moe_down1(const Down1Arg
             }
             float w0f, w1f;
             plane_weights(tid, mx / M1_QMAX, w0f, w1f);
-            y0 = (float)t[0] * w0f + (float)t[1] * w1f;
-            y1 = (float)t[2] * w0f + (float)t[3] * w1f;
+            y0 = fmaf((float)t[0], w0f, __fmul_rn((float)t[1], w1f));
+            y1 = fmaf((float)t[2], w0f, __fmul_rn((float)t[3], w1f));
             y0 += __shfl_xor_sync(0xffffffffu, y0, 1); y1 += __shfl_xor_sync(0xffffffffu, y1, 1);
             if (row0 + gid < a.D) y0 *= bf(a.shd_s[row0 + gid]);
             if (row0 + gid + 8 < a.D) y1 *= bf(a.shd_s[row0 + gid + 8]);

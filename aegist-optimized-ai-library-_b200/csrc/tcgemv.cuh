@@ -313,7 +313,7 @@ __global__ void __launch_bounds__((W + TC_EPI) * 32, 1) k_tcgemv(const GemvArgs 
                 for (int g = 0; g < NG; g++)
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
-                        float v = (float)c0[g][2 * h] * pw0[g] + (float)c0[g][2 * h + 1] * pw1[g];
+                        float v = fmaf((float)c0[g][2 * h], pw0[g], __fmul_rn((float)c0[g][2 * h + 1], pw1[g]));      // (spelt out: k_step1 has to round alike)
                         v += __shfl_xor_sync(0xffffffffu, v, 1);
                         const int b = 2 * g + (tid >> 1);
                         if ((tid & 1) == 0 && b < NB) pt[((size_t)b * W + ks) * 32 + rbk * 16 + gid + h * 8] = v;
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__((W + TC_EPI) * 32, 1) k_tcgemv(const GemvArgs 
                 float* out = sg.out + (size_t)(b0 + b) * sg.out_stride;
                 switch (sg.kind) {
                 case SEG_I8: out[row] = e0 * sA; break;
-                case SEG_I8_ACC: out[row] += e0 * sA; break;
+                case SEG_I8_ACC: out[row] = fmaf(e0, sA, out[row]); break;
                 case SEG_I8_SILU: out[row] = siluf_(e0 * sA); break;
                 case SEG_I8_ARGMAX: {
                     const float v0 = e0 * sA;

@@ -82,6 +82,7 @@ SYMBOLS = {
     "b2_set_router_bias": (_I, [_P, _I, _P]),
     "b2_debug_seek": (_I, [_P, _I]),
     "b2_launches_per_step": (_I, [_P]),
+    "b2_kernels_per_step": (_I, [_P]),
     "b2_debug_umma_launches": (C.c_long, []),
     "b2_debug_refuse_tensor_maps": (None, [_I]),
     "b2_step_bytes": (C.c_double, [_P]),
@@ -398,7 +399,11 @@ class HybridEngine:
         self._check(self._lib.b2_debug_seek(self._h, n))
 
     def launches_per_step(self) -> int:
+        """Stages of a step: a kernel launch each, or a stage of the one launch that runs a step of one sequence."""
         return self._lib.b2_launches_per_step(self._h)
+
+    def kernels_per_step(self) -> int:
+        return self._lib.b2_kernels_per_step(self._h)
 
     def step_bytes(self) -> float:
         return self._lib.b2_step_bytes(self._h)

@@ -381,7 +381,7 @@ def b64_measure(pkg, K: int, W: int, world: int, rank: int, local: int, dist, pe
         t = torch.tensor([e2e_s], device="cuda")
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         e2e_s = float(t.item())
-    n_launch = eng.launches_per_step()
+    n_launch = eng.kernels_per_step()
     nvlink = eng.ep_bytes_per_step() if world > 1 else 0
     eng.close()
     torch.cuda.empty_cache()
@@ -546,9 +546,10 @@ def run_ours(args):
     consistent = bool(abs(roles_sum_ms - ms / K) <= 0.10 * (ms / K))
     if not consistent:
         print(f"warning: the roles' in-graph times sum to {roles_sum_ms:.3f} ms, the timed step is {ms / K:.3f} ms", file=sys.stderr)
-    roof = {"bound": "hbm", "kernel": f"{name} ({E.HybridEngine.KERNELS_SMALL_BATCH[name]})", "achieved": achieved, "peak": peak,
+    one = eng.kernels_per_step() == 1                # a stage of the one launch that runs the step, or a launch
+    roof = {"bound": "hbm", "kernel": f"{name} ({'k_step1, its stage' if one else E.HybridEngine.KERNELS_SMALL_BATCH[name]})", "achieved": achieved, "peak": peak,
             "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
-            "traffic": NCU_DRAM_BYTES_PER_LAUNCH.get(name), "traffic_source": NCU_DRAM_SOURCE,
+            "traffic": None if one else NCU_DRAM_BYTES_PER_LAUNCH.get(name), "traffic_source": None if one else NCU_DRAM_SOURCE,
             "launches_per_step": dom["launches"], "bytes_per_launch": dom["bytes"] / max(dom["launches"], 1),
             "ms_per_launch": dom_us / 1e3 / max(dom["launches"], 1),
             "timing": "device global timer inside the CUDA graph of one decode step (b2_debug_trace_step); "
@@ -559,7 +560,7 @@ def run_ours(args):
             "ungraphed_events": {n: {"ms_per_step": round(v["ms"], 4), "GBps": round(v["bytes"] / max(v["ms"], 1e-9) / 1e6, 1),
                                      "launches": v["launches"], "kernel": E.HybridEngine.KERNELS_SMALL_BATCH[n]} for n, v in prof.items()}}
     cb = parity = b64 = None
-    n_launch = eng.launches_per_step()
+    n_launch = eng.kernels_per_step()
     eng.close()
     torch.cuda.empty_cache()
     if rank == 0 and world == 1 and not args.no_b64:

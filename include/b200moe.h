@@ -155,8 +155,10 @@ int b2_set_router_bias(b2_engine* e, int layer, const float* bias);
  * hold (zeros after loading) and the recurrent state is untouched. For timing a step at a given
  * context length; the logits that follow are not those of any real prompt. No reference counterpart. */
 int b2_debug_seek(b2_engine* e, int n);
-/* Number of kernel launches in one decode step (all sequences). */
+/* Stages of one decode step (all sequences): kernel launches, or the stages of the one persistent launch that runs a
+ * step of a single sequence; and how many kernels it launches. */
 int b2_launches_per_step(const b2_engine* e);
+int b2_kernels_per_step(const b2_engine* e);
 /* How many launches of the tcgen05 GEMM (k_umma) this process has enqueued so far, graph captures included: lets a
  * test see that the Blackwell tensor-core path, not a fall-back, is what ran. No counterpart in the reference. */
 long b2_debug_umma_launches(void);

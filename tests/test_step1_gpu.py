@@ -1,0 +1,117 @@
+"""A step of one sequence as one persistent launch (k_step1) against the same step as one launch per stage.
+
+DeltaNet, experts and head add in the same order on both ways, so a model without attention has the same bits. The attention cuts its
+context differently; each way is within 3e-4 of the oracle (test_kernel_edges), so they are within 6e-4 of one another (2e-3 each with
+the bf16 cache, whose newest values round alike but meet a hidden state that differs in its last bits)."""
+import importlib
+import threading
+
+import numpy as np
+import pytest
+
+gpu = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def E(pkg):
+    return importlib.import_module("b200moe.engine")
+
+
+def shape(pkg, name, layers):
+    """The widths the kernel is built for: d_model / output width of the mixers / key width / head width / expert width."""
+    if name == "full":
+        return pkg.HybridConfig.full(n_layers=layers)
+    cfg = pkg.HybridConfig.tiny() if name == "tiny" else pkg.HybridConfig.full(n_layers=layers)
+    if name == "narrow":                     # mixers as wide as the model
+        cfg.lin_k_heads, cfg.lin_v_heads, cfg.n_heads, cfg.head_dim, cfg.rotary_dim = 8, 16, 16, 128, 64
+    if name == "half":
+        cfg.d_model, cfg.expert_hidden, cfg.shared_hidden = 1024, 256, 256
+        cfg.lin_k_heads, cfg.lin_v_heads, cfg.n_heads, cfg.head_dim, cfg.rotary_dim = 8, 16, 16, 128, 32
+    cfg.n_layers = layers
+    cfg.layer_types = ["attn" if i % 4 == 3 else "delta" for i in range(layers)]
+    if name != "full":
+        cfg.vocab_size = 20008               # blocks' shares of the head that are no whole tiles
+    return cfg
+
+
+def pair(E, pkg, monkeypatch, cfg, kv, cap):
+    from b200moe import brain
+    dev = list(brain.random_brain(cfg, seed=1, device="cuda:0", vary_1d=True))
+    one = E.HybridEngine.from_tensors(cfg.to_dict(), dev, max_context=cap, device=0, batch=1, kv_dtype=kv)
+    monkeypatch.setenv("B2_NO_STEP1", "1")
+    many = E.HybridEngine.from_tensors(cfg.to_dict(), dev, max_context=cap, device=0, batch=1, kv_dtype=kv)
+    monkeypatch.delenv("B2_NO_STEP1")
+    assert one.kernels_per_step() == 1 and many.kernels_per_step() > cfg.n_layers
+    return one, many
+
+
+@gpu
+@pytest.mark.parametrize("name", ["tiny", "half", "narrow", "full"])
+def test_same_bits_without_attention(E, pkg, monkeypatch, name):
+    cfg = shape(pkg, name, 3)
+    one, many = pair(E, pkg, monkeypatch, cfg, E.KV_F32, 64)
+    for tok in np.random.default_rng(3).integers(0, cfg.vocab_size, 6):
+        a, b = (np.array(e.feed([int(tok)])) for e in (one, many))
+        assert np.array_equal(a, b)
+    for layer in range(cfg.n_layers):
+        for a, b in zip(one.router(layer, cfg.experts_active), many.router(layer, cfg.experts_active)):
+            assert np.array_equal(a, b), layer
+    assert np.array_equal(one.core_counts(cfg.n_layers, cfg.n_cores), many.core_counts(cfg.n_layers, cfg.n_cores))
+    one.close(); many.close()
+
+
+@gpu
+@pytest.mark.parametrize("kv", ["f32", "bf16"])
+@pytest.mark.parametrize("name,context", [("tiny", 1), ("tiny", 15), ("tiny", 2300), ("half", 1184), ("narrow", 17), ("full", 16), ("full", 63),
+                                          ("full", 64), ("full", 1183), ("full", 1185), ("full", 4800)])
+def test_attention_slices(E, pkg, monkeypatch, name, context, kv):
+    """Slices of 16 positions up to 16 x their number (74 of 2 KV heads, 148 of one), longer ones behind; page borders; a block's second pass
+    over its slice (more than two tiles of keys)."""
+    cfg = shape(pkg, name, 4)
+    one, many = pair(E, pkg, monkeypatch, cfg, E.KV_F32 if kv == "f32" else E.KV_BF16, context + 16)
+    ids = np.random.default_rng(context).integers(0, cfg.vocab_size, context)
+    for e in (one, many):
+        e.feed(ids[:-1] if context > 1 else ids, want_logits=False)
+    tol = 6e-4 if kv == "f32" else 4e-3
+    for tok in (5, 6, 7):
+        a, b = (np.array(e.feed([tok])) for e in (one, many))
+        assert np.isfinite(a).all() and np.abs(a - b).max() < tol
+    one.close(); many.close()
+
+
+@gpu
+def test_taps(E, pkg, monkeypatch):
+    """A layer that is tapped twice has one place in the launch's table: steps go by launches then, and back when the taps change."""
+    cfg = shape(pkg, "tiny", 3)
+    one, many = pair(E, pkg, monkeypatch, cfg, E.KV_F32, 64)
+    for layers in ([0, 2], [1, 1], [2]):
+        one.set_taps(layers); many.set_taps(layers)
+        assert (one.kernels_per_step() == 1) == (len(set(layers)) == len(layers))
+        a, b = (np.array(e.feed([9])) for e in (one, many))
+        assert np.array_equal(a, b) and np.array_equal(np.array(one.taps()), np.array(many.taps()))
+    one.close(); many.close()
+
+
+@gpu
+def test_engines_of_several_threads(E, pkg):
+    """Three engines on one device, each from its own thread: no launch may hold some SMs and wait for others."""
+    from b200moe import brain
+    cfg = shape(pkg, "tiny", 4)
+    dev = list(brain.random_brain(cfg, seed=1, device="cuda:0", vary_1d=True))
+    es = [E.HybridEngine.from_tensors(cfg.to_dict(), dev, max_context=512, device=0, batch=1, kv_dtype=E.KV_F32) for _ in range(3)]
+    want = []
+    for i, e in enumerate(es):
+        want.append(np.array(e.decode_greedy([i + 1], 100)[0]))
+        e.crop(0)
+    got = [None] * 3
+
+    def run(i):
+        got[i] = np.array(es[i].decode_greedy([i + 1], 100)[0])
+
+    ts = [threading.Thread(target=run, args=(i,)) for i in range(3)]
+    for t in ts: t.start()
+    for t in ts: t.join()
+    for w, g in zip(want, got):
+        assert np.array_equal(w, g)
+    for e in es:
+        e.close()
