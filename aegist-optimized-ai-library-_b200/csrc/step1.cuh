@@ -9,8 +9,8 @@
 //   * a value that other blocks need is stored once as 8 bytes, the fp32 value and the layer's tag, and a reader polls the very
 //     words it needs until they carry the tag: no counter, no fence, no grid-wide barrier between a value and its use;
 //   * every warp owns a slice of the contraction of all rows in the ring; one block barrier per stage where the slices meet.
-// 40 layers at context 4096: 1.44 ms a token, 1.62 ms as one launch per stage; at 190 (every token through the host) 1.45 and 1.71. A layer of
-// 50 MB takes 29 us, 8 of which HBM would need: the rest is the way of six dependent values from SM to SM (0.9 us each: a store and two
+// 40 layers at context 4096: 1.35 ms a token, 1.61 ms as one launch per stage; at 190 (every token through the host) 1.41 and 1.71. A layer of
+// 50 MB takes 27 us, 8 of which HBM would need: the rest is the way of six dependent values from SM to SM (0.9 us each: a store and two
 // polls of L2) and what lies between their coming and the products, in every warp.
 //
 // Every sum is added in the order and with the roundings of the kernels that run steps of two to five sequences, so that a sequence has
@@ -763,6 +763,8 @@ __global__ void __launch_bounds__(S1_THREADS, 1) k_step1(const __grid_constant__
     // where it is long. A warp holds the 256 values (a chunk) its slice lies in, eight to a lane
     constexpr int D = SD * 16, KO = SO * 16, S2 = D / 8, OSL = KO > 2048 ? 16 : 8, S3 = KO / OSL, NC = D / 256, NCO = KO / 256;
     constexpr int GE = D / 512;                   // gate/up: 64-code groups of an eighth of a row
+    constexpr int XP = D / 512;                   // values of a lane when all warps share a vector of D
+    static_assert(NC <= 8 && S1_WARPS % NC == 0 && (XP == 1 || XP % 2 == 0), "named barriers 3 .. 10, ll_wait");
     extern __shared__ __align__(128) unsigned char s1_smem[];
     unsigned char* ring = s1_smem;
     unsigned char* scratch_all = ring + (size_t)a.nst * a.stage_bytes;
@@ -1010,6 +1012,7 @@ __global__ void __launch_bounds__(S1_THREADS, 1) k_step1(const __grid_constant__
         pw0 = scale * (tid == 0 ? 1.0f : (tid == 1 ? 1.0f / 65536.0f : 0.f));
         pw1 = pw0 * (1.0f / 256.0f);
     };
+    auto out_chunk = [](int w) { return (OSL == 16 ? w : w >> 1) * S3 / 256; };      // of the mixers' output: the one warp w holds
     auto sum_of = [&](const float* p, int n) {    // one row's partial sums of n slices
         float s = 0.f;
 #pragma unroll
@@ -1043,11 +1046,22 @@ __global__ void __launch_bounds__(S1_THREADS, 1) k_step1(const __grid_constant__
             uint32_t nw[4];
             const int k = ck * 256 + lane * 8;
             ldg_words<4>((head ? a.norm : (moe ? ly.norm2 : ly.norm1)) + k, nw);
-            if (rd == 0) {
+            {
+                // a chunk's warps poll a part of it each and share it: 148 blocks' polls are bytes that L2 has to deliver (2.4 MB a look, 0.4 us)
+                float xp[XP];
+                const int kp = ck * 256 + (warp % (S1_WARPS / NC)) * 32 * XP + lane * XP;
+                if (rd == 0) {
 #pragma unroll
-                for (int i = 0; i < 8; i++) xv[i] = bf(a.embed[(size_t)s_blk.id * D + k + i]);
-            } else ll_wait<8>((moe ? set + a.o_xb : a.ll + (size_t)((l & 1) ^ 1) * a.ll_set + a.o_xa) + k, moe ? tag : tag - 1, true, xv, flag);
-            tr.pt(1);
+                    for (int i = 0; i < XP; i++) xp[i] = bf(a.embed[(size_t)s_blk.id * D + kp + i]);
+                } else ll_wait<XP>((moe ? set + a.o_xb : a.ll + (size_t)((l & 1) ^ 1) * a.ll_set + a.o_xa) + kp, moe ? tag : tag - 1, true, xp, flag);
+                tr.pt(1);
+#pragma unroll
+                for (int i = 0; i < XP; i++) xf_all[kp + i] = xp[i];
+                __syncwarp();
+                bar_sync(3 + ck, 32 * (S1_WARPS / NC));
+                const float4 x0 = *reinterpret_cast<const float4*>(xf_all + k), x1 = *reinterpret_cast<const float4*>(xf_all + k + 4);
+                xv[0] = x0.x; xv[1] = x0.y; xv[2] = x0.z; xv[3] = x0.w; xv[4] = x1.x; xv[5] = x1.y; xv[6] = x1.z; xv[7] = x1.w;
+            }
 #pragma unroll
             for (int i = 0; i < 8; i++) { ss = fmaf(xv[i], xv[i], ss); xv[i] *= 1.0f + ((i & 1) ? bfhi(nw[i / 2]) : bflo(nw[i / 2])); mx = fmaxf(mx, fabsf(xv[i])); }
             ss = warp_sum(ss);
@@ -1249,6 +1263,19 @@ __global__ void __launch_bounds__(S1_THREADS, 1) k_step1(const __grid_constant__
             constexpr int RPT = DK / 8;                         // state rows of a lane of the eight warps that hold the slab, as in k_delta_step
             const int nslab = a.DV / 32, ntask = a.HV * nslab;
             tr.in(3, ntask, blk < ntask);
+            // silu(z) for the out projection, in scratch, slices w and w + 1: warps that do not hold the state fetch them for all, so that the polls for
+            // the delta rule's output look at nothing else (9.5 MB a look with both; 0.4 us of a layer)
+            auto fetch_z = [&](int w) {
+                float z0[8], z1[8];
+                ll_wait2<8, 8>(set + a.o_z + out_chunk(w) * 256 + lane * 8, set + a.o_z + out_chunk(w + 1) * 256 + lane * 8, tag, true, z0, z1, flag);
+                float4 *t0 = reinterpret_cast<float4*>(scratch_all + w * SM::SCR) + 2 * lane, *t1 = reinterpret_cast<float4*>(scratch_all + (w + 1) * SM::SCR) + 2 * lane;
+                t0[0] = make_float4(z0[0], z0[1], z0[2], z0[3]);
+                t0[1] = make_float4(z0[4], z0[5], z0[6], z0[7]);
+                t1[0] = make_float4(z1[0], z1[1], z1[2], z1[3]);
+                t1[1] = make_float4(z1[4], z1[5], z1[6], z1[7]);
+            };
+            if (blk >= ntask && warp < 8) fetch_z(2 * warp);
+            if (blk >= ntask) s1_bar();
             for (int t = blk; t < ntask; t += G) {
                 const int col0 = (t % nslab) * 32, h = t / nslab;
                 float* S = ly.state + ((size_t)h * DK) * a.DV + col0 + lane;
@@ -1293,9 +1320,10 @@ __global__ void __launch_bounds__(S1_THREADS, 1) k_step1(const __grid_constant__
                     float v[1];
                     ll_wait<1>(set + a.o_bg + (lane & 1) * a.HV + h, tag, true, v, flag);
                     if (lane < 2) bs[lane] = lane ? expf(v[0]) : v[0];
-                }
+                } else if (warp >= 12 && t == blk) fetch_z(2 * (warp - 8));
                 s1_bar();
                 tr.pt(1);
+                if (warp >= 8 && warp < 12 && t == blk) fetch_z(2 * (warp - 8));
                 if (warp < 8) {
                     const float decay = bs[1];
                     float kv = 0.f;
@@ -1346,14 +1374,18 @@ __global__ void __launch_bounds__(S1_THREADS, 1) k_step1(const __grid_constant__
                 if (mine && ti >= tile && ti < tile + n) e0 = bf(reinterpret_cast<const uint16_t*>(rg.stage(ti - tile) + a.stage_bytes - S1_OPS)[(row0 & 7) + slot_row]);
                 tile += n;
             };
-            const int os = OSL == 16 ? warp : warp >> 1, opar = OSL == 16 ? -1 : warp & 1, oc = os * S3 / 256, k0 = oc * 256 + lane * 8;
+            const int os = OSL == 16 ? warp : warp >> 1, opar = OSL == 16 ? -1 : warp & 1, oc = out_chunk(warp), k0 = oc * 256 + lane * 8;
             float xv[8], mx = 0.f, pw0, pw1;
             if (!attn) {
                 // w * rmsnorm_DV(o) * silu(z) per value head (aegist/hybrid.py:133-147); a head is DV / 8 neighbouring lanes
                 float zv[8], ss = 0.f;
                 uint32_t gw[4];
                 ldg_words<4>(ly.n_a + k0 % a.DV, gw);
-                ll_wait2<8, 8>(set + a.o_og + k0, set + a.o_z + k0, tag, true, xv, zv, flag);
+                ll_wait<8>(set + a.o_og + k0, tag, true, xv, flag);
+                {
+                    const float4 *from = reinterpret_cast<const float4*>(scratch) + 2 * lane, z0 = from[0], z1 = from[1];
+                    zv[0] = z0.x; zv[1] = z0.y; zv[2] = z0.z; zv[3] = z0.w; zv[4] = z1.x; zv[5] = z1.y; zv[6] = z1.z; zv[7] = z1.w;
+                }
 #pragma unroll
                 for (int i = 0; i < 8; i++) ss = fmaf(xv[i], xv[i], ss);
                 for (int o = a.DV >> 4; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
