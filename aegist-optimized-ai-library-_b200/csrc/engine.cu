@@ -1576,8 +1576,10 @@ int b2_engine::feed_chunk(const uint32_t* ids, int T, bool want_head) {
 struct Step1Shape { int sd, so, dk, hd, gh; const void* kernel; int smem_rest; };
 #define S1_SHAPE(sd, so, dk, hd, gh) {sd, so, dk, hd, gh, (const void*)k_step1<sd, so, dk, hd, gh>, Step1Smem<sd, so, hd, gh>::TOTAL}
 // widths the kernel is built for: d_model / 16, the mixers' output width / 16, key width of the delta rule, head width, expert
-// hidden / 128
-static const Step1Shape STEP1_SHAPES[] = {S1_SHAPE(32, 32, 64, 128, 1), S1_SHAPE(64, 128, 128, 128, 2), S1_SHAPE(128, 128, 128, 128, 4), S1_SHAPE(128, 256, 128, 256, 4)};
+// hidden / 128. d_model from 1024 on: a stage takes 4 to 5 us whatever its width, which is what a launch of 512 values takes. Microseconds a
+// token of eight layers, one launch against a launch per stage: d_model 512 235, 226; 1024 222, 275 (its head has fewer rows); 2048
+// with mixers as wide 250, 290; with mixers of 4096 315, 368.
+static const Step1Shape STEP1_SHAPES[] = {S1_SHAPE(64, 128, 128, 128, 2), S1_SHAPE(128, 128, 128, 128, 4), S1_SHAPE(128, 256, 128, 256, 4)};
 
 // Rows of several matrices dealt out to G blocks in one go: block b owns the rows that start in its share of all bytes, in order, cut into
 // tiles of at most seg.maxn rows. False if a block gets more tiles than it has room for.

@@ -9,7 +9,7 @@
 //   * a value that other blocks need is stored once as 8 bytes, the fp32 value and the layer's tag, and a reader polls the very
 //     words it needs until they carry the tag: no counter, no fence, no grid-wide barrier between a value and its use;
 //   * every warp owns a slice of the contraction of all rows in the ring; one block barrier per stage where the slices meet.
-// 40 layers at context 4096: 1.35 ms a token, 1.61 ms as one launch per stage; at 190 (every token through the host) 1.41 and 1.71. A layer of
+// 40 layers at context 4096: 1.36 ms a token, 1.61 ms as one launch per stage; at 190 (every token through the host) 1.38 and 1.71. A layer of
 // 50 MB takes 27 us, 8 of which HBM would need: the rest is the way of six dependent values from SM to SM (0.9 us each: a store and two
 // polls of L2) and what lies between their coming and the products, in every warp.
 //
@@ -1320,10 +1320,10 @@ __global__ void __launch_bounds__(S1_THREADS, 1) k_step1(const __grid_constant__
                     float v[1];
                     ll_wait<1>(set + a.o_bg + (lane & 1) * a.HV + h, tag, true, v, flag);
                     if (lane < 2) bs[lane] = lane ? expf(v[0]) : v[0];
-                } else if (warp >= 12 && t == blk) fetch_z(2 * (warp - 8));
+                }
                 s1_bar();
                 tr.pt(1);
-                if (warp >= 8 && warp < 12 && t == blk) fetch_z(2 * (warp - 8));
+                if (warp >= 8 && t == blk) fetch_z(2 * (warp - 8));
                 if (warp < 8) {
                     const float decay = bs[1];
                     float kv = 0.f;

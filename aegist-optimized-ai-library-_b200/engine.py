@@ -413,6 +413,7 @@ class HybridEngine:
         return self._lib.b2_ep_bytes_per_step(self._h)
 
     # roles of the launches of a decode step; which kernel fills a role depends on the batch:
+    #   1 sequence: stages of k_step1 where the widths allow it; profile_step times the launches of 2-5 sequences instead
     #   1-5 sequences: k_tcgemv (in_proj, out_proj, head), k_moe_gu1, k_moe_down1
     #   6+ sequences:  k_prep_q + k_umma (tcgen05 GEMMs), k_group_picks + k_prep_q_slots + k_umma_q4 for the experts
     KERNEL_CLASSES = ("embed", "in_proj", "delta_step", "attention", "out_proj", "expert_gate_up", "expert_down", "head")

@@ -19,16 +19,12 @@ def E(pkg):
 
 def shape(pkg, name, layers):
     """The widths the kernel is built for: d_model / output width of the mixers / key width / head width / expert width."""
-    if name == "full":
-        return pkg.HybridConfig.full(n_layers=layers)
-    cfg = pkg.HybridConfig.tiny() if name == "tiny" else pkg.HybridConfig.full(n_layers=layers)
+    cfg = pkg.HybridConfig.full(n_layers=layers)
     if name == "narrow":                     # mixers as wide as the model
         cfg.lin_k_heads, cfg.lin_v_heads, cfg.n_heads, cfg.head_dim, cfg.rotary_dim = 8, 16, 16, 128, 64
     if name == "half":
         cfg.d_model, cfg.expert_hidden, cfg.shared_hidden = 1024, 256, 256
         cfg.lin_k_heads, cfg.lin_v_heads, cfg.n_heads, cfg.head_dim, cfg.rotary_dim = 8, 16, 16, 128, 32
-    cfg.n_layers = layers
-    cfg.layer_types = ["attn" if i % 4 == 3 else "delta" for i in range(layers)]
     if name != "full":
         cfg.vocab_size = 20008               # blocks' shares of the head that are no whole tiles
     return cfg
@@ -46,7 +42,7 @@ def pair(E, pkg, monkeypatch, cfg, kv, cap):
 
 
 @gpu
-@pytest.mark.parametrize("name", ["tiny", "half", "narrow", "full"])
+@pytest.mark.parametrize("name", ["half", "narrow", "full"])
 def test_same_bits_without_attention(E, pkg, monkeypatch, name):
     cfg = shape(pkg, name, 3)
     one, many = pair(E, pkg, monkeypatch, cfg, E.KV_F32, 64)
@@ -62,11 +58,11 @@ def test_same_bits_without_attention(E, pkg, monkeypatch, name):
 
 @gpu
 @pytest.mark.parametrize("kv", ["f32", "bf16"])
-@pytest.mark.parametrize("name,context", [("tiny", 1), ("tiny", 15), ("tiny", 2300), ("half", 1184), ("narrow", 17), ("full", 16), ("full", 63),
+@pytest.mark.parametrize("name,context", [("half", 1), ("half", 15), ("half", 1184), ("narrow", 17), ("full", 16), ("full", 63),
                                           ("full", 64), ("full", 1183), ("full", 1185), ("full", 4800)])
 def test_attention_slices(E, pkg, monkeypatch, name, context, kv):
-    """Slices of 16 positions up to 16 x their number (74 of 2 KV heads, 148 of one), longer ones behind; page borders; a block's second pass
-    over its slice (more than two tiles of keys)."""
+    """Slices of 16 positions up to 16 x 74 (blocks per KV head), longer ones behind; page borders; a block's second pass over its slice
+    (more than two tiles of keys)."""
     cfg = shape(pkg, name, 4)
     one, many = pair(E, pkg, monkeypatch, cfg, E.KV_F32 if kv == "f32" else E.KV_BF16, context + 16)
     ids = np.random.default_rng(context).integers(0, cfg.vocab_size, context)
@@ -80,9 +76,18 @@ def test_attention_slices(E, pkg, monkeypatch, name, context, kv):
 
 
 @gpu
+def test_narrow_model_keeps_its_launches(E, pkg):
+    from b200moe import brain
+    cfg = pkg.HybridConfig.tiny()
+    e = E.HybridEngine.from_tensors(cfg.to_dict(), brain.random_brain(cfg, seed=1, device="cuda:0"), max_context=64, device=0, batch=1, kv_dtype=E.KV_F32)
+    assert e.kernels_per_step() > cfg.n_layers
+    e.close()
+
+
+@gpu
 def test_taps(E, pkg, monkeypatch):
     """A layer that is tapped twice has one place in the launch's table: steps go by launches then, and back when the taps change."""
-    cfg = shape(pkg, "tiny", 3)
+    cfg = shape(pkg, "half", 3)
     one, many = pair(E, pkg, monkeypatch, cfg, E.KV_F32, 64)
     for layers in ([0, 2], [1, 1], [2]):
         one.set_taps(layers); many.set_taps(layers)
@@ -96,7 +101,7 @@ def test_taps(E, pkg, monkeypatch):
 def test_engines_of_several_threads(E, pkg):
     """Three engines on one device, each from its own thread: no launch may hold some SMs and wait for others."""
     from b200moe import brain
-    cfg = shape(pkg, "tiny", 4)
+    cfg = shape(pkg, "half", 4)
     dev = list(brain.random_brain(cfg, seed=1, device="cuda:0", vary_1d=True))
     es = [E.HybridEngine.from_tensors(cfg.to_dict(), dev, max_context=512, device=0, batch=1, kv_dtype=E.KV_F32) for _ in range(3)]
     want = []
