@@ -268,7 +268,7 @@ __device__ __forceinline__ void core_route_warp(const CoreRoute& cr, int t, int 
     const float ex = lane < k ? expf(myv - top) : 0.f;
     float sum = 0.f;
     for (int j = 0; j < k; j++) sum += __shfl_sync(0xffffffffu, ex, j);        // summed in pick order, as one thread would
-    if (lane < k) {
+    if (lane < k && mycore >= 0 && mycore < cr.n1 * cr.n2) {         // (scores that are no numbers leave no pick)
         cr.sel[(size_t)t * cr.k + lane] = mycore;
         cr.selw[(size_t)t * cr.k + lane] = ex / sum;
         atomicAdd(cr.counts + mycore, 1);
