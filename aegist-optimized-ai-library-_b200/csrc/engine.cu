@@ -1637,22 +1637,24 @@ static bool deal_spread(const std::vector<Step1Seg>& heavy, const std::vector<St
     return true;
 }
 
-// Decides whether steps of this engine run as one persistent launch, and lays out what that needs. Not an error if they do not.
-int b2_engine::plan_step1() {
-    const int G = nsm;
-    if (B != 1 || ep_world != 1 || live_cores > 0 || getenv("B2_NO_STEP1")) return 0;
+// Which rows every one of G blocks multiplies, and the copies that fetch them: host arithmetic on the widths. n1, n2: rows of the core engine's
+// tables (0, 0: this brain has none). False where the kernel is not built for the shape.
+struct Step1Plan {
+    const Step1Shape* sh = nullptr;
+    int n8, h8, hb, ho, hp, hs, stage;             // rows of an int8 tile; where the second half of a tile's rows begins, by matrix; bytes of a tile
+    std::vector<uint32_t> tiles;
+    std::vector<S1Copy> copies;
+};
+static bool lay_out_step1(const Cfg& c, int G, int n1, int n2, bool kv_f32, Step1Plan& p) {
     const int hr = c.RD / 2;
     const bool rope_ok = c.RD > 0 && c.RD <= c.HD && hr % std::max(1, c.HD / 32) == 0;
     if (c.G != 64 || c.CK != 4 || c.TOPK > 8 || c.E > 256 || c.E % 8 || c.SH % 32 || c.SH > 512 || c.I % 128 || !rope_ok || c.H % c.KV || c.H / c.KV > 8 || c.KV > G ||
         c.HV % std::max(c.HK, 1) || (c.DV != 64 && c.DV != 128) || c.H * c.HD != c.VD() || c.D < G || (c.D + G - 1) / G > 16 || c.TOPK * c.I < G ||
         (c.TOPK * c.I + G - 1) / G > 32 || (c.n1 + c.n2) % 2 || c.V < G || c.V >= 1 << 24 ||
-        c.V % 8 || c.C() % 8 || c.VD() % 8 || c.HV % 8 || (c.KV * c.HD) % 8 || c.SH % 8 || c.D % 8) return 0;       // (the last: 16-byte pieces of their scales)
-    const Step1Shape* sh = nullptr;
+        c.V % 8 || c.C() % 8 || c.VD() % 8 || c.HV % 8 || (c.KV * c.HD) % 8 || c.SH % 8 || c.D % 8) return false;       // (the last: 16-byte pieces of their scales)
     for (const Step1Shape& s : STEP1_SHAPES)
-        if (s.sd * 16 == c.D && s.so * 16 == c.VD() && s.dk == c.DK && s.hd == c.HD && s.gh * 128 == c.I) sh = &s;
-    if (!sh) return 0;
-    const int ns = G / c.KV, chunk = std::max(16, (cap + ns - 1) / ns);
-    if ((chunk + KV_PAGE - 1) / KV_PAGE + 1 > S1_PAGES) return 0;
+        if (s.sd * 16 == c.D && s.so * 16 == c.VD() && s.dk == c.DK && s.hd == c.HD && s.gh * 128 == c.I) p.sh = &s;
+    if (!p.sh) return false;
     // tiles: as many rows as make the longest share of the DeltaNet in-projections (the largest stage) a whole number of them
     const int VD = c.VD(), KO = VD, rd = (c.D + G - 1) / G, gp = (c.TOPK * c.I + G - 1) / G;
     const long u = ((long)c.C() + VD + 4L * c.HV + G - 1) / G;
@@ -1661,23 +1663,17 @@ int b2_engine::plan_step1() {
     const int h8 = s1_half_at(n8, c.D), hb = s1_half_at(nb, 2 * c.D), ho = s1_half_at(no, KO), hp = s1_half_at(np, c.D), hs = s1_half_at(rd, c.SH);
     const int stage = (std::max({h8 + n8 / 2 * c.D, hb + nb / 2 * 2 * c.D, ho + no / 2 * KO, 3 * hp + np / 2 * c.D, hs + rd / 2 * c.SH,
                                  gp * (c.D / 2) + 64, c.TOPK * s1_dn_stride(rd, c.I / 2), 16 * c.HD * (kv_f32 ? 4 : 2), 4 * s1_gsc_stride(c.D) + 2 * c.TOPK * s1_dsc_stride(c.I)}) + 15) / 16 * 16;
-    cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, sh->kernel) != cudaSuccess) { cudaGetLastError(); return 0; }
-    if (!s1_regs_suffice(fa.numRegs)) return 0;
-    const long room = 227 * 1024 - (long)fa.sharedSizeBytes - sh->smem_rest;
-    const int nst = (int)std::min<long>(S1_MAXST, room / (stage + S1_OPS));
-    if (nst < 5) return 0;         // the attention looks at two tiles of keys while their values are on their way, the experts at three of four
     std::vector<uint32_t> tiles((size_t)G * S1_TILES, S1_NONE);
     if (!deal_spread({{c.HV, 2, nb}, {c.HV, 2, nb}}, {{c.C(), 1, n8}, {VD, 1, n8}}, G, S1_IN_DELTA, tiles) ||
         !deal_tiles({{2 * c.H * c.HD, 1, n8}, {c.KV * c.HD, 1, n8}, {c.KV * c.HD, 1, n8}}, G, S1_IN_ATTN, tiles) ||
         !deal_tiles({{c.D, 1, no}}, G, S1_OUT, tiles) ||
-        !deal_tiles({{c.E, 1, nb}, {c.n1, 1, nb}, {c.n2, 1, nb}, {1, 1, nb}, {c.SH, 1, np}}, G, S1_MOE, tiles) ||
-        !deal_tiles({{c.D, 1, 16}}, G, S1_SHD, tiles)) return 0;
+        !deal_tiles({{c.E, 1, nb}, {n1, 1, nb}, {n2, 1, nb}, {1, 1, nb}, {c.SH, 1, np}}, G, S1_MOE, tiles) ||
+        !deal_tiles({{c.D, 1, 16}}, G, S1_SHD, tiles)) return false;
     // every block has its rows of the residual stream where the kernel expects them
     for (int b = 0; b < G; b++) {
         const uint32_t t = tiles[(size_t)b * S1_TILES + s1_at(S1_SHD)];
         const int r0 = (int)((long)b * c.D / G), r1 = (int)((long)(b + 1) * c.D / G);
-        if (t != s1_tile(0, r1 - r0, r0) || (int)(tiles[(size_t)b * S1_TILES + s1_at(S1_OUT)] & 0xffffff) != r0) return 0;
+        if (t != s1_tile(0, r1 - r0, r0) || (int)(tiles[(size_t)b * S1_TILES + s1_at(S1_OUT)] & 0xffffff) != r0) return false;
     }
     // the copies that fetch a tile: its two halves (four of a tile of gate-up pairs) and what the epilogue needs of its rows
     std::vector<S1Copy> copies((size_t)G * S1_TILES * S1_COPIES, S1Copy{0, 0});
@@ -1715,7 +1711,30 @@ int b2_engine::plan_step1() {
                 if (kind == S1_MOE && seg == 0) op(Q_BIAS, 4, 64);
                 if (pair) { op(S_GATE, 2, 0); op(S_UP, 2, 64); }
             }
-    if (!fits) return 0;
+    if (!fits) return false;
+    p.n8 = n8; p.h8 = h8; p.hb = hb; p.ho = ho; p.hp = hp; p.hs = hs; p.stage = stage;
+    p.tiles = std::move(tiles); p.copies = std::move(copies);
+    return true;
+}
+
+// Decides whether steps of this engine run as one persistent launch, and lays out what that needs. Not an error if they do not.
+int b2_engine::plan_step1() {
+    const int G = nsm;
+    if (B != 1 || ep_world != 1 || live_cores > 0 || getenv("B2_NO_STEP1")) return 0;
+    bool keys = false;
+    for (const LayerW& l : layers) keys = keys || l.key1;
+    const int n1 = keys ? c.n1 : 0, n2 = keys ? c.n2 : 0;
+    Step1Plan p;
+    if (!lay_out_step1(c, G, n1, n2, kv_f32, p)) return 0;
+    const Step1Shape* sh = p.sh;
+    const int ns = G / c.KV, chunk = std::max(16, (cap + ns - 1) / ns), stage = p.stage;
+    if ((chunk + KV_PAGE - 1) / KV_PAGE + 1 > S1_PAGES) return 0;
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, sh->kernel) != cudaSuccess) { cudaGetLastError(); return 0; }
+    if (!s1_regs_suffice(fa.numRegs)) return 0;
+    const long room = 227 * 1024 - (long)fa.sharedSizeBytes - sh->smem_rest;
+    const int nst = (int)std::min<long>(S1_MAXST, room / (stage + S1_OPS));
+    if (nst < 5) return 0;         // the attention looks at two tiles of keys while their values are on their way, the experts at three of four
     const size_t smem = (size_t)nst * (stage + S1_OPS) + sh->smem_rest;
     int per_sm = 0;
     if (cudaFuncSetAttribute(sh->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
@@ -1723,16 +1742,16 @@ int b2_engine::plan_step1() {
     Step1Args& a = s1.args;
     uint32_t at = 0;
     auto part = [&](uint32_t n) { const uint32_t o = at; at += (n + 15) / 16 * 16; return o; };
-    a.o_xa = part(c.D); a.o_xb = part(c.D); a.o_q = part(std::max(c.C(), (2 * c.H + 2 * c.KV) * c.HD)); a.o_z = part(VD); a.o_bg = part(2 * c.HV);
-    a.o_og = part(KO); a.o_rl = part(c.E); a.o_sa = part(c.SH); a.o_sg = part(1); a.o_act = part(c.TOPK * c.I);
+    a.o_xa = part(c.D); a.o_xb = part(c.D); a.o_q = part(std::max(c.C(), (2 * c.H + 2 * c.KV) * c.HD)); a.o_z = part(c.VD()); a.o_bg = part(2 * c.HV);
+    a.o_og = part(c.VD()); a.o_rl = part(c.E); a.o_sa = part(c.SH); a.o_sg = part(1); a.o_act = part(c.TOPK * c.I);
     a.ll_set = at;
     at *= 2;
-    a.o_ap = part(c.KV * ns * 8 * (c.HD + 2)); a.cs_words = (c.n1 + c.n2 + 15) / 16 * 16; a.o_cs = part(c.L * a.cs_words);
+    a.o_ap = part(c.KV * ns * 8 * (c.HD + 2)); a.cs_words = (n1 + n2 + 15) / 16 * 16; a.o_cs = part(c.L * a.cs_words);
     CU(dalloc(&s1.ll, at));
-    CU(dalloc(&s1.tiles, tiles.size(), false));
-    CU(cudaMemcpy(s1.tiles, tiles.data(), tiles.size() * 4, cudaMemcpyHostToDevice));
-    CU(dalloc(&s1.copies, copies.size(), false));
-    CU(cudaMemcpy(s1.copies, copies.data(), copies.size() * sizeof(S1Copy), cudaMemcpyHostToDevice));
+    CU(dalloc(&s1.tiles, p.tiles.size(), false));
+    CU(cudaMemcpy(s1.tiles, p.tiles.data(), p.tiles.size() * 4, cudaMemcpyHostToDevice));
+    CU(dalloc(&s1.copies, p.copies.size(), false));
+    CU(cudaMemcpy(s1.copies, p.copies.data(), p.copies.size() * sizeof(S1Copy), cudaMemcpyHostToDevice));
     CU(dalloc(&s1.epoch, 1));
     CU(dalloc(&s1.layers, c.L, false));
     if (G > head_grid) {                       // the arg-max' scratch: one place per block
@@ -1743,7 +1762,7 @@ int b2_engine::plan_step1() {
     a.layers = s1.layers; a.tiles = s1.tiles; a.embed = embed; a.norm = norm; a.head_w = lm_head.w; a.head_s = lm_head.s; a.logits = logits; a.x = x; a.ll = s1.ll;
     a.epoch = s1.epoch; a.rope_cos = rope_cos; a.rope_sin = rope_sin; a.page_table = page_table; a.scale = 1.0f / std::sqrt((float)c.HD); a.eps = c.eps;
     a.L = c.L; a.V = c.V; a.E = c.E; a.topk = c.TOPK; a.I = c.I; a.SH = c.SH; a.HK = c.HK; a.HV = c.HV; a.DV = c.DV; a.H = c.H; a.KV = c.KV; a.RD = c.RD; a.C = c.C();
-    a.n1 = c.n1; a.n2 = c.n2; a.cores_k = c.cores_active; a.kv_f32 = kv_f32; a.half_i8 = h8; a.half_bf = hb; a.half_out = ho; a.half_pair = hp; a.half_shd = hs; a.copies = s1.copies; a.kv_tile = std::min(64, stage / (c.HD * (kv_f32 ? 4 : 2))); a.head_rows = n8; a.nst = nst; a.stage_bytes = stage + S1_OPS;
+    a.n1 = n1; a.n2 = n2; a.cores_k = c.cores_active; a.kv_f32 = kv_f32; a.half_i8 = p.h8; a.half_bf = p.hb; a.half_out = p.ho; a.half_pair = p.hp; a.half_shd = p.hs; a.copies = s1.copies; a.kv_tile = std::min(64, stage / (c.HD * (kv_f32 ? 4 : 2))); a.head_rows = p.n8; a.nst = nst; a.stage_bytes = stage + S1_OPS;
     a.expert_bytes = c.expert_bytes(); a.off_gu_s = c.off_gu_s(); a.off_gu_m = c.off_gu_m(); a.off_dn_q = c.off_dn_q(); a.off_dn_s = c.off_dn_s(); a.off_dn_m = c.off_dn_m();
     a.cscore = cscore; a.csel = csel; a.cselw = cselw; a.part_val = part_val; a.part_idx = part_idx; a.next_tok = d_next; a.pos = d_pos; a.tok = d_tok;
     a.hist = TokHist{d_hist, cap, 1}; a.counter = d_counter; a.err = d_err;
@@ -1775,7 +1794,7 @@ int b2_engine::upload_step1() {
             t.n_a = l.gnorm; t.conv_w = l.conv; t.a_log = l.a_log; t.dt_bias = l.dt_bias;
             t.conv_state = conv + (size_t)l.slot * c.C() * 3; t.state = state + (size_t)l.slot * c.HV * c.DK * c.DV;
         }
-        t.w[5] = l.router; t.w[6] = l.key1 ? l.key1 : l.router; t.w[7] = l.key2 ? l.key2 : l.router; t.w[8] = l.sh_gw;      // without a core engine the key rows are not looked at
+        t.w[5] = l.router; t.w[6] = l.key1; t.w[7] = l.key2; t.w[8] = l.sh_gw;      // (a layer without keys among layers with them: nothing is copied)
         put(9, 4, l.sh_gate); put(10, 5, l.sh_up); put(11, 6, l.sh_down);
         t.norm1 = l.norm1; t.norm2 = l.norm2; t.bias = l.router_bias; t.experts = l.experts;
         t.counts = l.key1 ? d_counts + (size_t)i * c.n1 * c.n2 : nullptr;
@@ -2479,6 +2498,34 @@ double b2_ep_bytes_per_step(const b2_engine* e) {
     }
     const double back = peers * e->B * (c.TOPK + 1.0) * c.D * 4;         // pick outputs computed here, to their owners
     return c.L * (gather + back);
+}
+
+int b2_debug_step1_plan(const char* config_json, int sms, int has_keys, int kv_dtype, int64_t* out, int cap) {
+    b2_engine e;                       // (for its config only: no device is touched)
+    JValue j;
+    std::string err;
+    JParser parser(config_json, strlen(config_json));
+    if (!parser.parse(j, err) || e.parse_config(j) || sms < 1) return -1;
+    const Cfg& c = e.c;
+    Step1Plan p;
+    if (!lay_out_step1(c, sms, has_keys ? c.n1 : 0, has_keys ? c.n2 : 0, kv_dtype == B2_KV_F32, p)) return 0;
+    int n = 0;
+    for (int b = 0; b < sms; b++)
+        for (int kind = 0; kind < S1_KINDS; kind++)
+            for (int i = 0; i < s1_cap(kind); i++) {
+                const size_t ti = (size_t)b * S1_TILES + s1_at(kind) + i;
+                const uint32_t t = p.tiles[ti];
+                if (t == S1_NONE) break;
+                for (int k = 0; k < S1_COPIES; k++) {
+                    const S1Copy& y = p.copies[ti * S1_COPIES + k];
+                    if (!(y.what >> 16)) continue;
+                    const int64_t r[9] = {b, kind, (int64_t)(t >> 29), (int64_t)((t >> 24) & 31), (int64_t)(t & 0xffffff), (int64_t)(y.what & 31), (int64_t)y.from * 16,
+                                          (int64_t)(y.what >> 16) * 16, (int64_t)((y.what >> 5) & 2047) * 16 - p.stage};
+                    if (n < cap) std::copy(r, r + 9, out + (size_t)9 * n);
+                    n++;
+                }
+            }
+    return n;
 }
 
 int b2_debug_trace_step(b2_engine* e, unsigned long long* out, int cap_launches, int* n_launches) {

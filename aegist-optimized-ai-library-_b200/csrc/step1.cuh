@@ -920,7 +920,7 @@ __global__ void __launch_bounds__(S1_THREADS, 1) k_step1(const __grid_constant__
                     if (s_tiles[i] == S1_NONE) break;
                     const S1Copy c = s_copies[i * S1_COPIES + (lane & (S1_COPIES - 1))];
                     const char* src = (const char*)__shfl_sync(0xffffffffu, wp, c.what & 31u);
-                    issue(src + (size_t)c.from * 16u, lane < S1_COPIES && src ? (c.what >> 16) * 16u : 0u, ((c.what >> 5) & 2047u) * 16u);       // (a layer may have no router bias)
+                    issue(src + (size_t)c.from * 16u, lane < S1_COPIES && src ? (c.what >> 16) * 16u : 0u, ((c.what >> 5) & 2047u) * 16u);       // (a layer may have no core keys: nobody reads what its tiles then hold)
                 }
                 if (kind == S1_IN_ATTN) {
                     // this block's slice of the cache: keys of up to two tiles, then their values, and again. Rows of a page lie one after another; the

@@ -85,6 +85,7 @@ SYMBOLS = {
     "b2_kernels_per_step": (_I, [_P]),
     "b2_debug_umma_launches": (C.c_long, []),
     "b2_debug_refuse_tensor_maps": (None, [_I]),
+    "b2_debug_step1_plan": (_I, [C.c_char_p, _I, _I, _I, C.POINTER(C.c_int64), _I]),
     "b2_step_bytes": (C.c_double, [_P]),
     "b2_ep_bytes_per_step": (C.c_double, [_P]),
     "b2_profile_step": (_I, [_P, _I, C.POINTER(_F), C.POINTER(C.c_double), C.POINTER(_I)]),
@@ -433,6 +434,13 @@ class HybridEngine:
         n = C.c_int(0)
         self._check(self._lib.b2_debug_trace_step(self._h, buf, cap, C.byref(n)))
         return np.frombuffer(buf, dtype=np.uint64)[: 16 * n.value].reshape(n.value, 16).copy()
+
+
+def step1_plan(config: dict, sms: int = 148, has_keys: bool = True, kv_dtype: int = KV_F32):
+    """The copies of a layer's weights that the persistent step makes: an int64 array [copies][9] (see b2_debug_step1_plan)."""
+    buf = (C.c_int64 * (9 * 65536))()
+    n = load_library().b2_debug_step1_plan(json.dumps(config).encode(), sms, int(has_keys), kv_dtype, buf, 65536)
+    return np.frombuffer(buf, dtype=np.int64)[: 9 * max(n, 0)].reshape(-1, 9).copy()
 
 
 # --- sampler (aegist_rs/src/chat.rs:221-272) ----------------------------------------------------

@@ -162,6 +162,13 @@ int b2_kernels_per_step(const b2_engine* e);
 /* How many launches of the tcgen05 GEMM (k_umma) this process has enqueued so far, graph captures included: lets a
  * test see that the Blackwell tensor-core path, not a fall-back, is what ran. No counterpart in the reference. */
 long b2_debug_umma_launches(void);
+/* What the blocks of the persistent step of one sequence copy from the weights of a layer, for a GPU of `sms` SMs; no GPU is
+ * needed. A record is 9 words: block, stage (0 in-projections of a DeltaNet layer, 1 of attention, 2 out projection, 3 router,
+ * core keys and shared expert, 4 its down rows), matrix of the stage, rows of the tile, its first row, word of the layer's
+ * pointer, offset and bytes of the copy, and its place in the ring stage behind the rows (below 0: rows). Returns
+ * the number of records (`out` holds 9 * cap words), 0 where the step runs as launches, -1 for a config that no engine takes.
+ * No counterpart in the reference. */
+int b2_debug_step1_plan(const char* config_json, int sms, int has_keys, int kv_dtype, int64_t* out, int cap);
 /* While on, the calling thread's engines and operators are refused every tensor map, as a driver could: the kernels
  * that need none run instead. For tests of that fall-back. No counterpart in the reference. */
 void b2_debug_refuse_tensor_maps(int on);

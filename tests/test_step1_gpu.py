@@ -30,15 +30,49 @@ def shape(pkg, name, layers):
     return cfg
 
 
-def pair(E, pkg, monkeypatch, cfg, kv, cap):
+def pair(E, pkg, monkeypatch, cfg, kv, cap, keep=lambda name: True):
     from b200moe import brain
-    dev = list(brain.random_brain(cfg, seed=1, device="cuda:0", vary_1d=True))
+    dev = [t for t in brain.random_brain(cfg, seed=1, device="cuda:0", vary_1d=True) if keep(t[0])]
     one = E.HybridEngine.from_tensors(cfg.to_dict(), dev, max_context=cap, device=0, batch=1, kv_dtype=kv)
     monkeypatch.setenv("B2_NO_STEP1", "1")
     many = E.HybridEngine.from_tensors(cfg.to_dict(), dev, max_context=cap, device=0, batch=1, kv_dtype=kv)
     monkeypatch.delenv("B2_NO_STEP1")
     assert one.kernels_per_step() == 1 and many.kernels_per_step() > cfg.n_layers
     return one, many
+
+
+@pytest.mark.parametrize("keys", [True, False])
+@pytest.mark.parametrize("name", ["half", "narrow", "full", "few"])
+def test_every_row_is_copied_once_and_no_copy_leaves_its_tensor(E, pkg, name, keys):
+    """The layout of the persistent step, on the CPU. A brain without core engine tensors has no rows of theirs: with fewer experts than
+    keys ("few") copies in their place would read past the router."""
+    cfg = shape(pkg, "half" if name == "few" else name, 4)
+    if name == "few":
+        cfg.n_experts, cfg.core_grid = 64, (128, 128)
+    plan = E.step1_plan(cfg.to_dict(), 148, keys)
+    assert len(plan)
+    D, C, HV, VD, SH, En = cfg.d_model, cfg.conv_dim, cfg.lin_v_heads, cfg.lin_v_heads * cfg.lin_v_dim, cfg.shared_hidden, cfg.n_experts
+    q, kv = 2 * cfg.n_heads * cfg.head_dim, cfg.n_kv_heads * cfg.head_dim
+    n1, n2 = cfg.core_grid if keys else (0, 0)
+    # rows of a stage's matrices and bytes of a row; the tensors by the layer's pointer word, in bytes
+    rows = {0: [(HV, 2 * D), (HV, 2 * D), (C, D), (VD, D)], 1: [(q, D), (kv, D), (kv, D)], 2: [(D, VD)],
+            3: [(En, 2 * D), (n1, 2 * D), (n2, 2 * D), (1, 2 * D), (SH, D)], 4: [(D, SH)]}
+    first_ptr = {0: 0, 1: 0, 2: 4, 3: 5, 4: 11}
+    for kind, segs in rows.items():
+        size = {first_ptr[kind] + i: n * rb for i, (n, rb) in enumerate(segs)}
+        size.update({0: {12: 2 * C, 13: 2 * VD, 23: 8 * C, 24: 2 * HV, 25: 2 * HV, 26: 12 * C}, 1: {12: 2 * q, 13: 2 * kv, 14: 2 * kv},
+                     2: {15: 2 * D}, 3: {10: SH * D, 16: 2 * SH, 17: 2 * SH, 28: 4 * En}, 4: {18: 2 * D}}[kind])
+        of = plan[plan[:, 1] == kind]
+        for ptr, at, n in of[:, 5:8]:
+            assert at >= 0 and n > 0 and at % 16 == 0 and n % 16 == 0 and at + n <= size[ptr], (kind, ptr, at, n)
+        for i, (n, rb) in enumerate(segs):
+            for ptr in [first_ptr[kind] + i] + ([10] if (kind, i) == (3, 4) else []):
+                got = of[(of[:, 2] == i) & (of[:, 5] == ptr) & (of[:, 8] < 0)]
+                covered = np.zeros(n, np.int64)
+                for _, _, _, _, _, _, at, size_, _ in got:
+                    assert at % rb == 0 and size_ % rb == 0
+                    covered[at // rb:(at + size_) // rb] += 1
+                assert (covered == 1).all(), (kind, i, ptr)
 
 
 @gpu
@@ -53,6 +87,23 @@ def test_same_bits_without_attention(E, pkg, monkeypatch, name):
         for a, b in zip(one.router(layer, cfg.experts_active), many.router(layer, cfg.experts_active)):
             assert np.array_equal(a, b), layer
     assert np.array_equal(one.core_counts(cfg.n_layers, cfg.n_cores), many.core_counts(cfg.n_layers, cfg.n_cores))
+    one.close(); many.close()
+
+
+@gpu
+@pytest.mark.parametrize("which", ["none", "some layers"])
+def test_brain_without_core_engine(E, pkg, monkeypatch, which):
+    """Fewer experts than keys, and no keys: same bits as a launch per stage, and counts for the layers that have keys only."""
+    cfg = shape(pkg, "half", 3)
+    cfg.n_experts, cfg.core_grid = 64, (128, 128)
+    one, many = pair(E, pkg, monkeypatch, cfg, E.KV_F32, 64, lambda name: not (".engine.key" in name and (which == "none" or "blocks.1." in name)))
+    for tok in (5, 6, 7):
+        a, b = (np.array(e.feed([tok])) for e in (one, many))
+        assert np.array_equal(a, b)
+    counts = one.core_counts(cfg.n_layers, cfg.n_cores)
+    assert np.array_equal(counts, many.core_counts(cfg.n_layers, cfg.n_cores))
+    n = 3 * cfg.cores_active
+    assert counts.sum(1).tolist() == ([0, 0, 0] if which == "none" else [n, 0, n])
     one.close(); many.close()
 
 
