@@ -135,7 +135,7 @@ struct b2_engine {
 
     cudaStream_t stream = nullptr;
     cudaGraphExec_t graph = nullptr;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_other = nullptr;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_step = nullptr;
     int launches = 0;
 
     // state
@@ -320,7 +320,7 @@ b2_engine::~b2_engine() {
     if (h_pin) cudaFreeHost(h_pin);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
-    if (ev_other) cudaEventDestroy(ev_other);
+    if (ev_step) cudaEventDestroy(ev_step);
     for (cudaEvent_t e : prof_ev) cudaEventDestroy(e);
     if (comm && p_ncclCommDestroy) p_ncclCommDestroy(comm);
     if (stream) cudaStreamDestroy(stream);
@@ -631,7 +631,7 @@ int b2_engine::finish() {
     CU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CU(cudaEventCreate(&ev0));
     CU(cudaEventCreate(&ev1));
-    CU(cudaEventCreateWithFlags(&ev_other, cudaEventDisableTiming));
+    CU(cudaEventCreateWithFlags(&ev_step, cudaEventDisableTiming));
     CU(cudaDeviceSynchronize());
     finished = true;
     char buf[512];
@@ -1829,20 +1829,19 @@ int b2_engine::launch_step1(cudaStream_t st) {
 }
 
 // Persistent launches of two engines of a process must not hold half of a GPU's SMs each and wait for the other half: an engine that
-// follows another one on a device waits for what that one has enqueued so far. Nothing is added while one engine is used.
+// follows another one on a device waits for the event behind that one's last step. Every engine records its own: its stream belongs to its
+// thread, which may be capturing on it.
 static std::mutex g_step1_mutex;
 static std::map<int, b2_engine*> g_step1_last;          // device -> the engine whose step was launched last
 cudaError_t b2_engine::run_graph(cudaGraphExec_t g) {
     if (!use_step1()) return cudaGraphLaunch(g, stream);
     std::lock_guard<std::mutex> lock(g_step1_mutex);
     b2_engine*& last = g_step1_last[device];
-    if (last && last != this) {
-        cudaError_t e = cudaEventRecord(ev_other, last->stream);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, ev_other, 0);
-        if (e != cudaSuccess) return e;
-    }
+    cudaError_t e = last && last != this ? cudaStreamWaitEvent(stream, last->ev_step, 0) : cudaSuccess;
+    if (e == cudaSuccess) e = cudaGraphLaunch(g, stream);
+    if (e != cudaSuccess) return e;
     last = this;
-    return cudaGraphLaunch(g, stream);
+    return cudaEventRecord(ev_step, stream);
 }
 static void leave_step1(b2_engine* e) {
     if (!e->s1.layers) return;

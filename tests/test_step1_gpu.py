@@ -5,6 +5,7 @@ context differently; each way is within 3e-4 of the oracle (test_kernel_edges), 
 the bf16 cache, whose newest values round alike but meet a hidden state that differs in its last bits)."""
 import importlib
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -171,3 +172,37 @@ def test_engines_of_several_threads(E, pkg):
         assert np.array_equal(w, g)
     for e in es:
         e.close()
+
+
+@gpu
+def test_taps_change_beside_another_engine(E, pkg):
+    """An engine captures its step anew whenever its taps change; another engine that follows its steps has nothing to do with that."""
+    from b200moe import brain
+    cfg = shape(pkg, "half", 4)
+    dev = list(brain.random_brain(cfg, seed=1, device="cuda:0", vary_1d=True))
+    a, b = (E.HybridEngine.from_tensors(cfg.to_dict(), dev, max_context=64, device=0, batch=1, kv_dtype=E.KV_F32) for _ in range(2))
+    want = np.array(b.feed([3]))
+    errors, done = [], threading.Event()
+
+    def taps():
+        try:
+            while not done.is_set():
+                a.crop(0)
+                a.set_taps([0])
+                a.feed([1])
+                a.set_taps([1, 1])               # captured as many launches, which takes longer than one
+        except E.EngineError as x:
+            errors.append(x)
+
+    t = threading.Thread(target=taps)
+    t.start()
+    try:
+        for pause in np.random.default_rng(0).uniform(0, 3e-4, 1000):
+            b.crop(0)
+            assert np.array_equal(np.array(b.feed([3])), want)
+            time.sleep(pause)
+    finally:
+        done.set()
+        t.join()
+    assert not errors
+    a.close(); b.close()
