@@ -206,3 +206,26 @@ def test_taps_change_beside_another_engine(E, pkg):
         t.join()
     assert not errors
     a.close(); b.close()
+
+
+@gpu
+def test_a_step_beside_a_long_loop_has_its_turn(E, pkg):
+    """One step of an engine, asked for while another one is in a greedy loop of 3000 (about 0.6 s): it comes after the few steps that the loop has
+    queued, not after the loop."""
+    from b200moe import brain
+    cfg = shape(pkg, "half", 4)
+    dev = list(brain.random_brain(cfg, seed=1, device="cuda:0", vary_1d=True))
+    a, b = (E.HybridEngine.from_tensors(cfg.to_dict(), dev, max_context=3200, device=0, batch=1, kv_dtype=E.KV_F32) for _ in range(2))
+    want = np.array(a.decode_greedy([1], 3000)[0])
+    a.crop(0)
+    got = []
+    t = threading.Thread(target=lambda: got.append((np.array(a.decode_greedy([1], 3000)[0]), time.perf_counter())))
+    t0 = time.perf_counter()
+    t.start()
+    time.sleep(0.05)
+    b.feed([3])
+    fed = time.perf_counter()
+    t.join()
+    assert np.array_equal(got[0][0], want)
+    assert fed - t0 < 0.25 * (got[0][1] - t0)
+    a.close(); b.close()
