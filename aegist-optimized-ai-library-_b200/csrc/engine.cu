@@ -1742,7 +1742,8 @@ int b2_engine::plan_step1() {
     if (nst < 5) return 0;         // the attention looks at two tiles of keys while their values are on their way, the experts at three of four
     const size_t smem = (size_t)nst * (stage + S1_OPS) + sh->smem_rest;
     int per_sm = 0;
-    if (cudaFuncSetAttribute(sh->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+    // (the limit is the kernel's, not this engine's, and rings differ between engines: always all there is)
+    if (cudaFuncSetAttribute(sh->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sh->kernel, S1_THREADS, smem) != cudaSuccess || per_sm < 1) { cudaGetLastError(); return 0; }
     Step1Args& a = s1.args;
     uint32_t at = 0;

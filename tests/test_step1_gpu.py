@@ -150,6 +150,23 @@ def test_taps(E, pkg, monkeypatch):
 
 
 @gpu
+def test_another_engine_with_a_smaller_ring(E, pkg):
+    """The shared memory of the launch depends on more than the widths it is built for; an engine keeps its own when another one is opened."""
+    from b200moe import brain
+    cfg, less = shape(pkg, "full", 2), shape(pkg, "full", 2)
+    less.experts_active = 4
+    dev = list(brain.random_brain(cfg, seed=1, device="cuda:0", vary_1d=True))
+    a, b = (E.HybridEngine.from_tensors(c.to_dict(), dev, max_context=64, device=0, batch=1, kv_dtype=E.KV_F32) for c in (cfg, less))
+    assert a.kernels_per_step() == b.kernels_per_step() == 1
+    want = np.array(a.feed([7]))
+    a.set_taps([0])                      # captured again
+    a.crop(0)
+    assert np.array_equal(np.array(a.feed([7])), want)
+    b.feed([7])
+    a.close(); b.close()
+
+
+@gpu
 def test_engines_of_several_threads(E, pkg):
     """Three engines on one device, each from its own thread: no launch may hold some SMs and wait for others."""
     from b200moe import brain
