@@ -194,12 +194,13 @@ struct Seg {
 // The core engine (CoreEngine.forward, aegist/model.py:214-224; the routing half of cores_apply,
 // aegist_rs/kernels/aegist.cu:283-322): two score tables of n1 and n2 entries address n1 * n2 switchable cores. The k
 // best of each table, the k1 * k2 sums of their pairs, the k best sums (ties to the earlier one), softmax over those.
-// Every pick is tallied in counts[core] (Lm::core_counts); picks and weights are kept for the live cores' kernel.
+// Every pick is tallied in counts[core] (Lm::core_counts); picks and weights are kept for the live cores' kernel. Scores that are no numbers
+// (or -inf) are not picked: where fewer than k sums are left, the picks behind them are -1.
 struct CoreRoute {
     const float* score;      // [T][n1 + n2] the two tables' scores of every token (null: this brain has no core engine)
     int n1, n2, k;
     int* counts;             // [n1 * n2] of this layer
-    int* sel;                // [T][k]
+    int* sel;                // [T][k], -1: no pick
     float* selw;             // [T][k]
 };
 // one warp per token; n1 <= 128, n2 <= 128, k <= 8. Everything stays in registers (lane r holds the r-th pick of a
@@ -228,7 +229,8 @@ __device__ __forceinline__ void core_route_warp(const CoreRoute& cr, int t, int 
                 const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
                 if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
             }
-            if (lane == r) { if (tab) { pv1 = bv; pi1 = bi; } else { pv0 = bv; pi0 = bi; } }
+            const int found = bi < n ? bi : 0;       // (0 with a score of -inf: none is left that is a number)
+            if (lane == r) { if (tab) { pv1 = bv; pi1 = found; } else { pv0 = bv; pi0 = found; } }
             if ((bi & 31) == lane) {
                 const int j = bi >> 5;
                 if (j == 0) m0 = -INFINITY; else if (j == 1) m1 = -INFINITY; else if (j == 2) m2 = -INFINITY; else m3 = -INFINITY;
@@ -245,14 +247,14 @@ __device__ __forceinline__ void core_route_warp(const CoreRoute& cr, int t, int 
         const float va1 = __shfl_sync(0xffffffffu, pv0, a1 & 31), vb1 = __shfl_sync(0xffffffffu, pv1, b1 & 31);
         const int ia0 = __shfl_sync(0xffffffffu, pi0, a0 & 31), ib0 = __shfl_sync(0xffffffffu, pi1, b0 & 31);
         const int ia1 = __shfl_sync(0xffffffffu, pi0, a1 & 31), ib1 = __shfl_sync(0xffffffffu, pi1, b1 & 31);
-        c0 = lane < nc ? va0 + vb0 : -INFINITY; core0 = ia0 * cr.n2 + ib0;
-        c1 = lane + 32 < nc ? va1 + vb1 : -INFINITY; core1 = ia1 * cr.n2 + ib1;
+        c0 = lane < nc && va0 + vb0 > -INFINITY ? va0 + vb0 : -INFINITY; core0 = ia0 * cr.n2 + ib0;      // (a sum that is no number is no candidate)
+        c1 = lane + 32 < nc && va1 + vb1 > -INFINITY ? va1 + vb1 : -INFINITY; core1 = ia1 * cr.n2 + ib1;
     }
     float myv = 0.f;
-    int mycore = 0;
+    int mycore = -1;
     for (int j = 0; j < k; j++) {            // the j-th best sum goes to lane j; ties to the earlier candidate
         float bv = c0;
-        int bc = lane;
+        int bc = c0 > -INFINITY ? lane : 0x7fffffff;
         if (c1 > bv) { bv = c1; bc = lane + 32; }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -261,17 +263,17 @@ __device__ __forceinline__ void core_route_warp(const CoreRoute& cr, int t, int 
             if (ov > bv || (ov == bv && oc < bc)) { bv = ov; bc = oc; }
         }
         const int core = __shfl_sync(0xffffffffu, (bc >> 5) ? core1 : core0, bc & 31);
-        if (lane == j) { myv = bv; mycore = core; }
+        if (lane == j) { myv = bv; mycore = bc < nc ? core : -1; }
         if (lane == (bc & 31)) { if (bc >> 5) c1 = -INFINITY; else c0 = -INFINITY; }
     }
     const float top = __shfl_sync(0xffffffffu, myv, 0);
     const float ex = lane < k ? expf(myv - top) : 0.f;
     float sum = 0.f;
     for (int j = 0; j < k; j++) sum += __shfl_sync(0xffffffffu, ex, j);        // summed in pick order, as one thread would
-    if (lane < k && mycore >= 0 && mycore < cr.n1 * cr.n2) {         // (scores that are no numbers leave no pick)
+    if (lane < cr.k) {
         cr.sel[(size_t)t * cr.k + lane] = mycore;
-        cr.selw[(size_t)t * cr.k + lane] = ex / sum;
-        atomicAdd(cr.counts + mycore, 1);
+        cr.selw[(size_t)t * cr.k + lane] = mycore < 0 ? 0.f : ex / sum;
+        if (mycore >= 0) atomicAdd(cr.counts + mycore, 1);
     }
 }
 
@@ -1497,7 +1499,7 @@ __global__ void __launch_bounds__(256) k_cores_live(const CoresLiveArgs a) {
     for (int j = 0; j < 8; j++) acc[j] = 0.f;
     __syncthreads();
     for (int c = 0; c < a.k; c++) {
-        const int li = a.live[a.sel[(size_t)t * a.k + c]];
+        const int core = a.sel[(size_t)t * a.k + c], li = core < 0 ? -1 : a.live[core];
         if (li < 0) continue;        // the same for the whole block
         const uint16_t* G = a.cg + (size_t)li * a.D * a.r;
         const uint16_t* U = a.cu + (size_t)li * a.D * a.r;

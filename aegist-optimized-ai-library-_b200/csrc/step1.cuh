@@ -491,18 +491,19 @@ __device__ __forceinline__ void s1_core_route(const Step1Args& a, int* counts, i
                 const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
                 if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
             }
-            if (lane == r) { if (tab) { qv = bv; qi = bi; } else { pv = bv; pi = bi; } }
-            if ((bi & 31) == lane) taken |= 1u << (bi >> 5);
+            const bool found = bi < n;            // (no score is left that is a number)
+            if (lane == r) { if (tab) { qv = bv; qi = found ? bi : 0; } else { pv = bv; pi = found ? bi : 0; } }
+            if (found && (bi & 31) == lane) taken |= 1u << (bi >> 5);
         }
     }
     // the sums of all pairs, candidate c = a k1 + b in lane c & 31; the best ones in turn, ties to the earlier one
     uint32_t taken = 0u;
     float myv = 0.f;
-    int mycore = 0;
+    int mycore = -1;
 #pragma unroll 1
     for (int j = 0; j < k; j++) {
         float bv = -INFINITY;
-        int bc = 0x7fffffff, core = 0;
+        int bc = 0x7fffffff, core = -1;
 #pragma unroll 1
         for (int h = 0; h < 2; h++) {
             const int c = lane + 32 * h, x = c / k1, y = c - x * k1;
@@ -517,17 +518,17 @@ __device__ __forceinline__ void s1_core_route(const Step1Args& a, int* counts, i
             if (ov > bv || (ov == bv && oc < bc)) { bv = ov; bc = oc; core = od; }
         }
         if (lane == j) { myv = bv; mycore = core; }
-        if ((bc & 31) == lane) taken |= 1u << (bc >> 5);
+        if (bc < nc && (bc & 31) == lane) taken |= 1u << (bc >> 5);
     }
     const float best = __shfl_sync(0xffffffffu, myv, 0);
     const float ex = lane < k ? expf(myv - best) : 0.f;
     float sum = 0.f;
 #pragma unroll 1
     for (int j = 0; j < k; j++) sum += __shfl_sync(0xffffffffu, ex, j);        // in pick order
-    if (lane < k && mycore >= 0 && mycore < a.n1 * a.n2) {           // (scores that are no numbers leave no pick)
+    if (lane < a.cores_k) {
         a.csel[lane] = mycore;
-        a.cselw[lane] = ex / sum;
-        atomicAdd(counts + mycore, 1);
+        a.cselw[lane] = mycore < 0 ? 0.f : ex / sum;
+        if (mycore >= 0) atomicAdd(counts + mycore, 1);
     }
 }
 

@@ -150,6 +150,45 @@ def test_taps(E, pkg, monkeypatch):
 
 
 @gpu
+@pytest.mark.parametrize("rows1,rows2", [(0, 0), (3, 0), (1, 1), (1, 3), (3, 2)])
+def test_core_scores_that_are_no_numbers(E, pkg, monkeypatch, rows1, rows2):
+    """Key rows of NaN, but for the first few of each table: a token's picks are different cores of the others, as many as there are, in a
+    step of one sequence, of several and of a prompt."""
+    from b200moe import brain
+    cfg = shape(pkg, "half", 2)
+    cfg.cores_active = 4
+    dev = list(brain.random_brain(cfg, seed=1, device="cuda:0", vary_1d=True))
+    for name, _, t in dev:
+        if ".engine.key" in name:
+            t[rows1 if "key1" in name else rows2:] = float("nan")
+    make = lambda batch: E.HybridEngine.from_tensors(cfg.to_dict(), dev, max_context=64, device=0, batch=batch, kv_dtype=E.KV_F32)
+    one, some, many = make(1), make(3), make(8)
+    monkeypatch.setenv("B2_NO_STEP1", "1")
+    stages = make(1)
+    assert one.kernels_per_step() == 1 and stages.kernels_per_step() > 1
+    allowed = np.zeros((cfg.core_grid[0], cfg.core_grid[1]), bool)
+    allowed[:rows1, :rows2] = True
+
+    def check(e, tokens):
+        counts = e.core_counts(cfg.n_layers, cfg.n_cores)
+        assert (counts.sum(1) == tokens * min(cfg.cores_active, rows1 * rows2)).all()
+        assert counts.max() <= tokens and not counts[:, ~allowed.ravel()].any()
+        e.reset_counts()
+
+    for e in (one, stages):
+        e.feed([5])
+        e.feed([6])
+        check(e, 2)
+        e.feed(np.arange(40))
+        check(e, 40)
+    for e, batch in ((some, 3), (many, 8)):
+        e.feed_batch(np.arange(batch))
+        check(e, batch)
+    for e in (one, some, many, stages):
+        e.close()
+
+
+@gpu
 def test_another_engine_with_a_smaller_ring(E, pkg):
     """The shared memory of the launch depends on more than the widths it is built for; an engine keeps its own when another one is opened."""
     from b200moe import brain
