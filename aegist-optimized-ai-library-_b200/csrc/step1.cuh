@@ -355,9 +355,11 @@ __device__ __forceinline__ float sum32(const float (&v)[8]) {
 }
 
 // Softmax over up to 256 logits (eight neighbouring ones in each lane that `has` some) and the topk <= 8 largest in descending order, ties to the lower
-// index (aegist/hybrid.py:641-645); picks and probabilities into top and topv. A probability is positive, so its bits order like an
-// integer. A lane sorts its own and a round is one reduction over the lanes' first ones; where two probabilities are equal (which the
-// number of lanes that won a round shows) the rounds are made again by index.
+// index (aegist/hybrid.py:641-645); picks and probabilities into top and topv. A positive float's bits order like an integer's. A lane
+// sorts its own exponentials and a round is one reduction over the lanes' first ones. The division keeps their order, but for what it
+// rounds to one value: so only the picks and the best one left are divided, a lane each (256 divisions in one warp cost 0.6 us a layer),
+// and where two of those, or two exponentials (which the number of lanes that won a round shows), are equal, all are divided and the
+// rounds are made again by index.
 __device__ __forceinline__ void s1_route(float (&lg)[8], bool has, int topk, int lane, int* top, float* topv) {
     uint32_t key[8];
     int ex[8];
@@ -373,14 +375,8 @@ __device__ __forceinline__ void s1_route(float (&lg)[8], bool has, int topk, int
     const float s32 = sum32(lg);                  // of experts 32 w .. 32 w + 31, w = lane / 4
 #pragma unroll
     for (int w = 0; w < 8; w++) sum += __shfl_sync(0xffffffffu, s32, 4 * w);
-    const float inv = __frcp_rn(sum);
-    uint32_t p[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const float q = lg[i] * inv;
-        p[i] = has ? __float_as_uint(fmaf(fmaf(-q, sum, lg[i]), inv, q)) + 1u : 0u;       // the quotient, rounded once
-        key[i] = p[i];
-    }
+    for (int i = 0; i < 8; i++) key[i] = has ? __float_as_uint(lg[i]) + 1u : 0u;
     // a network of 19 exchanges; the order of equal ones is left open
 #define S1_CX(i, j) { const bool w = key[j] > key[i]; const uint32_t k = w ? key[i] : key[j]; key[i] = w ? key[j] : key[i]; key[j] = k; const int e = w ? ex[i] : ex[j]; ex[i] = w ? ex[j] : ex[i]; ex[j] = e; }
     S1_CX(0, 2) S1_CX(1, 3) S1_CX(4, 6) S1_CX(5, 7)
@@ -394,23 +390,31 @@ __device__ __forceinline__ void s1_route(float (&lg)[8], bool has, int topk, int
 #pragma unroll
     for (int i = 0; i < 8; i++) order |= (uint32_t)ex[i] << (3 * i);
     int wins = 0;
-    bool equal = false;
+    uint32_t mine = 0u;                           // lane r: the key of round r; lane topk: of the best one left
 #pragma unroll
     for (int r = 0; r < 8; r++)
         if (r < topk) {
             const uint32_t m = __reduce_max_sync(0xffffffffu, key[0]);
             const bool w = key[0] == m;
             sts_if(w, (void*)(top + r), (uint32_t)lane * 8u + (order & 7u));
-            sts_if(w, (void*)(topv + r), m - 1u);
+            if (lane == r) mine = m;
             wins += w ? 1 : 0;
-            equal = equal || (w && key[1] == m);
             order = w ? order >> 3 : order;
 #pragma unroll
             for (int i = 0; i < 7 - r; i++) key[i] = w ? key[i + 1] : key[i];
             key[7 - r] = w ? 0u : key[7 - r];
         }
-    if (__reduce_add_sync(0xffffffffu, (unsigned)wins) == (unsigned)topk && !__any_sync(0xffffffffu, equal)) return;
+    {
+        const uint32_t m = __reduce_max_sync(0xffffffffu, key[0]);
+        if (lane == topk) mine = m;
+    }
+    const uint32_t prob = mine ? __float_as_uint(__uint_as_float(mine - 1u) / sum) + 1u : 0u, next = __shfl_down_sync(0xffffffffu, prob, 1);
+    sts_if(lane < topk, (void*)(topv + lane), prob - 1u);
+    if (__reduce_add_sync(0xffffffffu, (unsigned)wins) == (unsigned)topk && !__any_sync(0xffffffffu, lane < topk && prob == next)) return;
     __syncwarp();
+    uint32_t p[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) p[i] = has ? __float_as_uint(lg[i] / sum) + 1u : 0u;
 #pragma unroll 1
     for (int r = 0; r < topk; r++) {
         uint32_t bk = p[0];

@@ -92,6 +92,35 @@ def test_same_bits_without_attention(E, pkg, monkeypatch, name):
 
 
 @gpu
+def test_routes_of_small_probabilities(E, pkg, monkeypatch):
+    """Picks down to probabilities that are subnormal or 0, where ranks and weights hang on how the softmax is divided: the same picks and bits
+    as a launch per stage."""
+    cfg = shape(pkg, "half", 1)
+    one, many = pair(E, pkg, monkeypatch, cfg, E.KV_F32, 64)
+    rng = np.random.default_rng(0)
+    for tok in range(40):
+        bias = np.full(cfg.n_experts, -200, np.float32)
+        top = rng.permutation(cfg.n_experts)[:12]
+        bias[top] = -rng.uniform(0, 110, 12)
+        bias[top[0]] = 0
+        for e in (one, many):
+            e.set_router_bias(0, bias)
+            e.feed([tok])
+        for a, b in zip(one.router(0, cfg.experts_active), many.router(0, cfg.experts_active)):
+            assert np.array_equal(a, b)
+    for at, value in ((slice(3, None), -np.inf), (slice(7, 8), np.inf), (slice(9, 10), np.nan)):
+        bias = np.zeros(cfg.n_experts, np.float32)
+        bias[at] = value
+        for e in (one, many):
+            e.crop(0)
+            e.set_router_bias(0, bias)
+            e.feed([1])
+        for a, b in zip(one.router(0, cfg.experts_active), many.router(0, cfg.experts_active)):
+            assert np.array_equal(a, b, equal_nan=True)
+    one.close(); many.close()
+
+
+@gpu
 @pytest.mark.parametrize("which", ["none", "some layers"])
 def test_brain_without_core_engine(E, pkg, monkeypatch, which):
     """Fewer experts than keys, and no keys: same bits as a launch per stage, and counts for the layers that have keys only."""
