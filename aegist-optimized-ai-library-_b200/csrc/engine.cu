@@ -1241,7 +1241,7 @@ static cudaError_t launch_moe1(const Cfg& c, const float* rlogits, const float* 
 // and only when chunk_head is set).
 int b2_engine::enqueue_step(cudaStream_t st, bool count, int chunk_T, bool chunk_head) {
     if (chunk_T == 0 && use_step1()) {
-        if (count) launches = s1.stages;
+        if (count) launches = 1;
         return launch_step1(st);
     }
     int n = 0;
@@ -2490,7 +2490,8 @@ int b2_set_router_bias(b2_engine* e, int layer, const float* bias) {
 }
 
 int b2_launches_per_step(const b2_engine* e) { return e ? e->launches : 0; }
-int b2_kernels_per_step(const b2_engine* e) { return !e ? 0 : (e->use_step1() ? 1 : e->launches); }
+int b2_kernels_per_step(const b2_engine* e) { return b2_launches_per_step(e); }
+int b2_stages_per_step(const b2_engine* e) { return !e ? 0 : (e->use_step1() ? e->s1.stages : e->launches); }
 long b2_debug_umma_launches(void) { return g_umma_launches; }
 void b2_debug_refuse_tensor_maps(int on) { g_refuse_maps = on != 0; }
 

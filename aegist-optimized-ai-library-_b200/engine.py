@@ -83,6 +83,7 @@ SYMBOLS = {
     "b2_debug_seek": (_I, [_P, _I]),
     "b2_launches_per_step": (_I, [_P]),
     "b2_kernels_per_step": (_I, [_P]),
+    "b2_stages_per_step": (_I, [_P]),
     "b2_debug_umma_launches": (C.c_long, []),
     "b2_debug_refuse_tensor_maps": (None, [_I]),
     "b2_debug_step1_plan": (_I, [C.c_char_p, _I, _I, _I, C.POINTER(C.c_int64), _I]),
@@ -400,11 +401,14 @@ class HybridEngine:
         self._check(self._lib.b2_debug_seek(self._h, n))
 
     def launches_per_step(self) -> int:
-        """Stages of a step: a kernel launch each, or a stage of the one launch that runs a step of one sequence."""
+        """Kernels that a step launches: 1 where a step of one sequence runs as one persistent launch."""
         return self._lib.b2_launches_per_step(self._h)
 
-    def kernels_per_step(self) -> int:
-        return self._lib.b2_kernels_per_step(self._h)
+    kernels_per_step = launches_per_step
+
+    def stages_per_step(self) -> int:
+        """Rows of a step's timeline: its launches, or the stages inside the one launch."""
+        return self._lib.b2_stages_per_step(self._h)
 
     def step_bytes(self) -> float:
         return self._lib.b2_step_bytes(self._h)
@@ -423,13 +427,14 @@ class HybridEngine:
                            "expert_down": "k_moe_down1", "head": "k_tcgemv"}
 
     def profile_step(self, iters: int = 8) -> dict:
-        """Per kernel class: mean ms per step, algorithmic bytes per step, launches per step."""
+        """Per kernel class: mean ms per step, algorithmic bytes per step, launches per step; of the kernels of a launch per
+        stage, also where steps run as one persistent launch."""
         ms, by, ln = (C.c_float * 8)(), (C.c_double * 8)(), (C.c_int * 8)()
         self._check(self._lib.b2_profile_step(self._h, iters, ms, by, ln))
         return {n: {"ms": ms[i], "bytes": by[i], "launches": ln[i]} for i, n in enumerate(self.KERNEL_CLASSES)}
 
     def trace_step(self, cap: int = 4096):
-        """Timeline of one graph-run decode step: a uint64 array [launches][16] (see b2_debug_trace_step)."""
+        """Timeline of one graph-run decode step: a uint64 array [stages_per_step()][16] (see b2_debug_trace_step)."""
         buf = (C.c_uint64 * (16 * cap))()
         n = C.c_int(0)
         self._check(self._lib.b2_debug_trace_step(self._h, buf, cap, C.byref(n)))

@@ -279,13 +279,15 @@ def run_profile_case(args):
     toks, ms = eng.decode_greedy(toks[-1], args.steps)
     if rank == 0:
         print(json.dumps({"profile_case": True, "layers": args.profile_case, "batch": batch, "gpus": world, "context": ctx, "steps": args.steps,
-                          "ms_per_step": ms / args.steps, "launches_per_step": eng.launches_per_step(), "note": "not a bench value"}), flush=True)
+                          "ms_per_step": ms / args.steps, "launches_per_step": eng.launches_per_step(), "stages_per_step": eng.stages_per_step(), "note": "not a bench value"}), flush=True)
     if args.timeline:
         # the step as the CUDA graph runs it: per launch, microseconds on the device global timer relative to the
         # first launch, and block 0's own progress (SM cycle counter at the sampled clock) at its points 1..7
         names = {1: "k_tcgemv", 3: "k_delta_step", 5: "k_moe_gu1", 6: "k_moe_down1", 7: "k_attn(_mma)", 8: "k_attn_merge", 9: "k_prep_x",
                  10: "k_mma_i8", 11: "k_group_picks", 12: "k_mma_q4", 13: "k_ep_combine", 14: "k_umma", 15: "k_prep_q", 16: "k_umma_q4",
                  17: "k_prep_q_slots", 18: "k_ep_push_records", 19: "k_ep_push_outputs", 20: "k_ep_wait"}
+        if eng.launches_per_step() == 1:     # the stages of the persistent step
+            names = {1: "matrices", 3: "delta rule", 5: "gate/up", 6: "down", 7: "attention", 8: "merge"}
         eng.trace_step()                     # every rank steps (the exchange is collective); rank 0 prints its own timeline
         t = eng.trace_step().astype(np.int64)
         ghz = args.timeline_ghz
@@ -381,7 +383,7 @@ def b64_measure(pkg, K: int, W: int, world: int, rank: int, local: int, dist, pe
         t = torch.tensor([e2e_s], device="cuda")
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         e2e_s = float(t.item())
-    n_launch = eng.kernels_per_step()
+    n_launch = eng.launches_per_step()
     nvlink = eng.ep_bytes_per_step() if world > 1 else 0
     eng.close()
     torch.cuda.empty_cache()
@@ -546,7 +548,7 @@ def run_ours(args):
     consistent = bool(abs(roles_sum_ms - ms / K) <= 0.10 * (ms / K))
     if not consistent:
         print(f"warning: the roles' in-graph times sum to {roles_sum_ms:.3f} ms, the timed step is {ms / K:.3f} ms", file=sys.stderr)
-    one = eng.kernels_per_step() == 1                # a stage of the one launch that runs the step, or a launch
+    one = eng.launches_per_step() == 1               # a stage of the one launch that runs the step, or a launch
     roof = {"bound": "hbm", "kernel": f"{name} ({'k_step1, its stage' if one else E.HybridEngine.KERNELS_SMALL_BATCH[name]})", "achieved": achieved, "peak": peak,
             "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
             "traffic": None if one else NCU_DRAM_BYTES_PER_LAUNCH.get(name), "traffic_source": None if one else NCU_DRAM_SOURCE,
@@ -560,7 +562,7 @@ def run_ours(args):
             "ungraphed_events": {n: {"ms_per_step": round(v["ms"], 4), "GBps": round(v["bytes"] / max(v["ms"], 1e-9) / 1e6, 1),
                                      "launches": v["launches"], "kernel": E.HybridEngine.KERNELS_SMALL_BATCH[n]} for n, v in prof.items()}}
     cb = parity = b64 = None
-    n_launch = eng.kernels_per_step()
+    n_launch = eng.launches_per_step()
     eng.close()
     torch.cuda.empty_cache()
     if rank == 0 and world == 1 and not args.no_b64:

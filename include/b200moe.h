@@ -155,10 +155,12 @@ int b2_set_router_bias(b2_engine* e, int layer, const float* bias);
  * hold (zeros after loading) and the recurrent state is untouched. For timing a step at a given
  * context length; the logits that follow are not those of any real prompt. No reference counterpart. */
 int b2_debug_seek(b2_engine* e, int n);
-/* Stages of one decode step (all sequences): kernel launches, or the stages of the one persistent launch that runs a
- * step of a single sequence; and how many kernels it launches. */
+/* Kernels that one decode step (all sequences) launches: 1 where a step of a single sequence runs as one persistent launch
+ * (b2_kernels_per_step is another name for it); and the stages of a step, the rows of its timeline: its launches, or
+ * the stages inside the one launch. */
 int b2_launches_per_step(const b2_engine* e);
 int b2_kernels_per_step(const b2_engine* e);
+int b2_stages_per_step(const b2_engine* e);
 /* How many launches of the tcgen05 GEMM (k_umma) this process has enqueued so far, graph captures included: lets a
  * test see that the Blackwell tensor-core path, not a fall-back, is what ran. No counterpart in the reference. */
 long b2_debug_umma_launches(void);
@@ -180,14 +182,15 @@ double b2_step_bytes(const b2_engine* e);
  * event after every launch, and report per kernel class the mean device time per step (ms), the
  * algorithmic bytes per step and the launches per step. Classes: 0 embedding gather, 1 norm + GEMV
  * groups, 2 DeltaNet step, 3 attention, 4 output projections, 5 expert gate/up, 6 expert down +
- * shared down, 7 head. */
+ * shared down, 7 head. Steps that otherwise run as one persistent launch are taken apart for this: the kernels of a launch
+ * per stage are what is timed (b2_debug_trace_step shows the stages of the one launch). */
 int b2_profile_step(b2_engine* e, int iters, float ms[8], double bytes[8], int launches[8]);
 /* Bytes this GPU sends to its peers in one decode step of an expert-parallel engine (0 on one GPU): the per-layer
  * records (all-gather) and the pick outputs computed here for other GPUs' sequences. No counterpart in the reference. */
 double b2_ep_bytes_per_step(const b2_engine* e);
 
 /* Timeline of one decode step as the CUDA graph runs it (debugging aid, no reference counterpart; the step
- * feeds the current tokens and advances the length by one). Per launch 16 words: [0] first block entered and
+ * feeds the current tokens and advances the length by one). Per launch, or stage of a persistent one, 16 words: [0] first block entered and
  * [4] last block left, in ns of the GPU's global timer; [5] kernel code (1 GEMV, 3 DeltaNet step, 5 expert
  * gate/up, 6 expert down, 7 attention, 8 attention merge; 0 = a kernel that records nothing); [6] a shape hint
  * (rows of the first matrix, or the grid); [8] the SM cycle counter of block 0 when it entered and [9]..[15]

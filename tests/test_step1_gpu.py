@@ -166,6 +166,21 @@ def test_narrow_model_keeps_its_launches(E, pkg):
 
 
 @gpu
+def test_timeline(E, pkg):
+    """One launch, and a row of the timeline for each of its stages: six of a DeltaNet layer, seven of attention, the head."""
+    from b200moe import brain
+    cfg = shape(pkg, "half", 4)
+    e = E.HybridEngine.from_tensors(cfg.to_dict(), brain.random_brain(cfg, seed=1, device="cuda:0"), max_context=64, device=0, batch=1, kv_dtype=E.KV_F32)
+    e.feed([1, 2, 3])
+    t = e.trace_step().astype(np.int64)
+    assert e.launches_per_step() == 1 and e.stages_per_step() == 3 * 6 + 7 + 1 and t.shape == (26, 16) and e.length() == 4
+    delta, attn = [1, 3, 1, 1, 5, 6], [1, 7, 8, 1, 1, 5, 6]          # in-projections, mixer (and merge), out, router, gate/up, down
+    assert t[:, 5].tolist() == 3 * delta + attn + [1]
+    assert (t[:, 4] > t[:, 0]).all() and (np.diff(t[:, 4]) > 0).all()      # a stage ends after it began, and after the one before
+    e.close()
+
+
+@gpu
 def test_taps(E, pkg, monkeypatch):
     """A layer that is tapped twice has one place in the launch's table: steps go by launches then, and back when the taps change."""
     cfg = shape(pkg, "half", 3)
