@@ -20,6 +20,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -692,10 +693,22 @@ static cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
     return launch_kc(1, kernel, grid, block, smem, st, args...);
 }
 
+// The limit belongs to the kernel on its device, and engines of several threads ask for different sizes: always all there is, once.
 template <typename F>
 static cudaError_t opt_in_smem(F* f, size_t bytes) {
     if (bytes <= 32 * 1024) return cudaSuccess;        // the 48 KB that need no opting in hold the kernel's static arrays too
-    return cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    static std::mutex mutex;
+    static std::set<std::pair<int, const void*>> known;
+    int device;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mutex);
+    if (known.count({device, (const void*)f})) return cudaSuccess;
+    cudaFuncAttributes fa;
+    e = cudaFuncGetAttributes(&fa, (const void*)f);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes);
+    if (e == cudaSuccess) known.insert({device, (const void*)f});
+    return e;
 }
 
 // k_mma_i8 over `passes` groups of MM_TOK sequences. A grid that gives an SM at most one block (the out projections,
@@ -1742,8 +1755,7 @@ int b2_engine::plan_step1() {
     if (nst < 5) return 0;         // the attention looks at two tiles of keys while their values are on their way, the experts at three of four
     const size_t smem = (size_t)nst * (stage + S1_OPS) + sh->smem_rest;
     int per_sm = 0;
-    // (the limit is the kernel's, not this engine's, and rings differ between engines: always all there is)
-    if (cudaFuncSetAttribute(sh->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes) != cudaSuccess ||
+    if (opt_in_smem(sh->kernel, smem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sh->kernel, S1_THREADS, smem) != cudaSuccess || per_sm < 1) { cudaGetLastError(); return 0; }
     Step1Args& a = s1.args;
     uint32_t at = 0;

@@ -1,0 +1,49 @@
+"""Engines of one process, each used by a thread of its own (include/b200moe.h), while one of them captures its step anew again and again
+as its taps change."""
+import contextlib
+import importlib
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def E(pkg):
+    return importlib.import_module("b200moe.engine")
+
+
+@contextlib.contextmanager
+def captures(e):
+    errors, done = [], threading.Event()
+
+    def taps():
+        try:
+            while not done.is_set():
+                e.set_taps([0])
+                e.set_taps([1, 2])
+        except Exception as x:
+            errors.append(x)
+
+    t = threading.Thread(target=taps)
+    t.start()
+    try:
+        yield
+    finally:
+        done.set()
+        t.join()
+    assert not errors, errors
+
+
+def test_prompts_beside_captures(E, tiny_path):
+    """The kernels' limit of shared memory is one for all threads: no launch lowers it for another one's."""
+    a, b = (E.HybridEngine.load(tiny_path, max_context=1024) for _ in range(2))
+    lengths = (40, 333, 40, 700, 17) * 20
+    want = {n: np.array(a.feed(np.arange(n))) for n in set(lengths) if a.crop(0) == 0}
+    with captures(b):
+        for n in lengths:
+            a.crop(0)
+            assert np.array_equal(np.array(a.feed(np.arange(n))), want[n])
+    a.close(); b.close()
