@@ -638,7 +638,9 @@ int b2_engine::finish() {
     CU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CU(cudaEventCreate(&ev0));
     CU(cudaEventCreate(&ev1));
-    CU(cudaDeviceSynchronize());
+    // what was loaded came over the default stream, which the engine's does not wait for. (A wait for the whole device would also be for streams
+    // that other threads capture on, which is an error here and breaks their captures)
+    CU(cudaStreamSynchronize(cudaStreamLegacy));
     finished = true;
     char buf[512];
     size_t kv_bytes = 2 * kv_elems * kvb;
@@ -1575,7 +1577,7 @@ int b2_engine::ensure_chunk_bufs(int T) {
     }
     total = 0;
     for (auto& part : parts) { *part.first = pc.arena + total; total += (part.second + align - 1) / align * align; }
-    CU(cudaDeviceSynchronize());         // the buffers' zeroes (default stream) before the engine's stream uses them
+    CU(cudaStreamSynchronize(cudaStreamLegacy));         // the buffers' zeroes (default stream) before the engine's stream uses them
     pc.W = W;
     return 0;
 }

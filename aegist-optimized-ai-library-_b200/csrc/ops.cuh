@@ -165,7 +165,7 @@ int b2_moe_create(int device, const b2_moe_weights* w, int max_tokens, b2_moe** 
     OPCU(cudaMallocHost((void**)&m->h_err, sizeof(int)));
     OPCU(cudaMallocHost((void**)&m->h_in, (size_t)T * c.D * 4));
     OPCU(cudaMallocHost((void**)&m->h_out, (size_t)T * (c.D + 2 * c.TOPK) * 4));
-    OPCU(cudaDeviceSynchronize());           // the buffers' zeroes (default stream) before the operator's stream uses them
+    OPCU(cudaStreamSynchronize(cudaStreamLegacy));           // the buffers' zeroes (default stream) before the operator's stream uses them
     OPCU(cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking));
     OPCU(cudaEventCreate(&m->e0)); OPCU(cudaEventCreate(&m->e1));
     return 0;

@@ -47,3 +47,17 @@ def test_prompts_beside_captures(E, tiny_path):
             a.crop(0)
             assert np.array_equal(np.array(a.feed(np.arange(n))), want[n])
     a.close(); b.close()
+
+
+def test_opening_beside_captures(E, tiny_path):
+    """Opening and closing an engine, and its first prompt, wait for what they have begun, not for the device with other threads' streams."""
+    b = E.HybridEngine.load(tiny_path, max_context=64)
+    want = None
+    with captures(b):
+        for _ in range(20):
+            a = E.HybridEngine.load(tiny_path, max_context=256)
+            got = np.array(a.feed(np.arange(100)))
+            want = got if want is None else want
+            assert np.array_equal(got, want)
+            a.close()
+    b.close()
