@@ -447,6 +447,7 @@ int b2_engine::qw(const std::string& prefix, int n, int k, QWd* out) {
     return 0;
 }
 
+// (zeroed on the default stream: whoever uses it on another one waits for that first)
 template <typename T>
 static cudaError_t dalloc(T** p, size_t n, bool zero = true) {
     cudaError_t e = cudaMalloc((void**)p, std::max<size_t>(n * sizeof(T), 16));
@@ -638,9 +639,6 @@ int b2_engine::finish() {
     CU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CU(cudaEventCreate(&ev0));
     CU(cudaEventCreate(&ev1));
-    // what was loaded came over the default stream, which the engine's does not wait for. (A wait for the whole device would also be for streams
-    // that other threads capture on, which is an error here and breaks their captures)
-    CU(cudaStreamSynchronize(cudaStreamLegacy));
     finished = true;
     char buf[512];
     size_t kv_bytes = 2 * kv_elems * kvb;
@@ -648,8 +646,11 @@ int b2_engine::finish() {
              gpu_name.c_str(), weight_bytes / 1e9, c.L * per, c.L * c.E, ep_world > 1 ? " on this rank" : "", live_cores, cap, B,
              kv_f32 ? "fp32" : "bf16", kv_bytes / 1e9);
     desc = buf;
+    if (ep_world == 1 && plan_step1()) return 1;
+    // everything so far came over the default stream, which the engine's does not wait for. (A wait for the whole device would also be for streams
+    // that other threads capture on, which is an error here and breaks their captures)
+    CU(cudaStreamSynchronize(cudaStreamLegacy));
     if (ep_world > 1) return 0;   // the step graph holds NCCL calls: it is built by b2_ep_init
-    if (plan_step1()) return 1;
     return build_graph();
 }
 
@@ -1826,7 +1827,8 @@ int b2_engine::upload_step1() {
             if (tap_layers[j] == i) { t.tap = tap_buf + j * (size_t)c.D; taps++; }
         if (taps > 1) s1.off = true;
     }
-    CU(cudaMemcpy(s1.layers, tab.data(), tab.size() * sizeof(Step1Layer), cudaMemcpyHostToDevice));
+    CU(cudaMemcpyAsync(s1.layers, tab.data(), tab.size() * sizeof(Step1Layer), cudaMemcpyHostToDevice, stream));       // (the steps' own stream)
+    CU(cudaStreamSynchronize(stream));
     return 0;
 }
 
@@ -2408,7 +2410,7 @@ int b2_load_state(b2_engine* e, const char* path, uint32_t* toks_out, int cap_to
     for (auto& pc : e->state_pieces(n)) {
         buf.resize(pc.bytes);
         if (fread(buf.data(), 1, pc.bytes, f) != pc.bytes) { fclose(f); e->reset_state(); return e->fail("%s: truncated", path); }
-        if (cudaMemcpy(pc.p, buf.data(), pc.bytes, cudaMemcpyHostToDevice) != cudaSuccess) { fclose(f); cudaGetLastError(); e->reset_state(); return e->fail("%s: upload failed", path); }
+        if (cudaMemcpyAsync(pc.p, buf.data(), pc.bytes, cudaMemcpyHostToDevice, e->stream) != cudaSuccess || cudaStreamSynchronize(e->stream) != cudaSuccess) { fclose(f); cudaGetLastError(); e->reset_state(); return e->fail("%s: upload failed", path); }
     }
     fclose(f);
     k_fill_i32<<<1, 32, 0, e->stream>>>(e->d_pos, n, 1);
@@ -2437,7 +2439,10 @@ int b2_set_taps(b2_engine* e, const int* layers, int n) {
     cudaFree(e->tap_buf);
     e->tap_buf = nullptr;
     e->tap_layers.assign(layers, layers + n);
-    if (n) CUE(dalloc(&e->tap_buf, (size_t)n * e->B * e->c.D));
+    if (n) {
+        CUE(dalloc(&e->tap_buf, (size_t)n * e->B * e->c.D, false));
+        CUE(cudaMemsetAsync(e->tap_buf, 0, (size_t)n * e->B * e->c.D * sizeof(float), e->stream));
+    }
     return e->build_graph();
 }
 
@@ -2496,10 +2501,10 @@ int b2_set_router_bias(b2_engine* e, int layer, const float* bias) {
     if (!e || !e->finished) return 1;
     if (layer < 0 || layer >= e->c.L) return e->fail("layer %d out of range", layer);
     CUE(cudaSetDevice(e->device));
-    CUE(cudaStreamSynchronize(e->stream));
     LayerW& l = e->layers[layer];
-    if (!bias) CUE(cudaMemset(l.router_bias, 0, (size_t)e->c.E * 4));
-    else CUE(cudaMemcpy(l.router_bias, bias, (size_t)e->c.E * 4, cudaMemcpyHostToDevice));
+    if (!bias) CUE(cudaMemsetAsync(l.router_bias, 0, (size_t)e->c.E * 4, e->stream));
+    else CUE(cudaMemcpyAsync(l.router_bias, bias, (size_t)e->c.E * 4, cudaMemcpyHostToDevice, e->stream));
+    CUE(cudaStreamSynchronize(e->stream));
     return 0;
 }
 

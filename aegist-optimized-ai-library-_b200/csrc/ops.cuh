@@ -260,6 +260,7 @@ int b2_delta_create(int device, int batch, int heads, int dk, int dv, const floa
     OPCU(dalloc(&d->y, (size_t)batch * C)); OPCU(dalloc(&d->g, (size_t)batch * heads)); OPCU(dalloc(&d->beta, (size_t)batch * heads));
     OPCU(dalloc(&d->o, (size_t)batch * heads * dv));
     d->pack.resize((size_t)batch * C);
+    OPCU(cudaStreamSynchronize(cudaStreamLegacy));           // state and zeroes (default stream) before the operator's stream uses them
     OPCU(cudaStreamCreateWithFlags(&d->st, cudaStreamNonBlocking));
     OPCU(cudaEventCreate(&d->e0)); OPCU(cudaEventCreate(&d->e1));
     return 0;
