@@ -655,12 +655,13 @@ int b2_engine::finish() {
 }
 
 
-static int g_launch_count = 0;   // kernels launched so far (a step's count is the difference)
+static thread_local int g_launch_count = 0;   // kernels that this thread has launched so far (a step's count is the difference)
 
 // Step timeline (b2_debug_trace_step): while g_trace_base is set, the launch with index i since g_trace_first
-// gets the slot g_trace_base + 16 i in its argument struct (structs with a `trace` member; null otherwise).
-static unsigned long long* g_trace_base = nullptr;
-static int g_trace_first = 0;
+// gets the slot g_trace_base + 16 i in its argument struct (structs with a `trace` member; null otherwise). A thread's own: another
+// engine's capture meanwhile must not take slots, nor keep pointers to them.
+static thread_local unsigned long long* g_trace_base = nullptr;
+static thread_local int g_trace_first = 0;
 constexpr int TRACE_MAX_LAUNCHES = 4096;
 template <typename T>
 static auto with_trace(const T& a, int) -> decltype((void)a.trace, T()) {

@@ -61,3 +61,12 @@ def test_opening_beside_captures(E, tiny_path):
             assert np.array_equal(got, want)
             a.close()
     b.close()
+
+
+def test_timeline_beside_captures(E, tiny_path):
+    """The slots of a timeline go to the launches of the thread that asked for it."""
+    a, b = (E.HybridEngine.load(tiny_path, max_context=256) for _ in range(2))
+    with captures(b):
+        rows = {a.trace_step().shape[0] for _ in range(200)}
+    assert rows == {a.stages_per_step()} and a.launches_per_step() == a.stages_per_step()
+    b.close(); a.close()
