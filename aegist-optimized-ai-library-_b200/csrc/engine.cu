@@ -1787,7 +1787,7 @@ int b2_engine::plan_step1() {
     a.n1 = n1; a.n2 = n2; a.cores_k = c.cores_active; a.kv_f32 = kv_f32; a.half_i8 = p.h8; a.half_bf = p.hb; a.half_out = p.ho; a.half_pair = p.hp; a.half_shd = p.hs; a.copies = s1.copies; a.kv_tile = std::min(64, stage / (c.HD * (kv_f32 ? 4 : 2))); a.head_rows = p.n8; a.nst = nst; a.stage_bytes = stage + S1_OPS;
     a.expert_bytes = c.expert_bytes(); a.off_gu_s = c.off_gu_s(); a.off_gu_m = c.off_gu_m(); a.off_dn_q = c.off_dn_q(); a.off_dn_s = c.off_dn_s(); a.off_dn_m = c.off_dn_m();
     a.cscore = cscore; a.csel = csel; a.cselw = cselw; a.part_val = part_val; a.part_idx = part_idx; a.next_tok = d_next; a.pos = d_pos; a.tok = d_tok;
-    a.hist = TokHist{d_hist, cap, 1}; a.counter = d_counter; a.err = d_err;
+    a.hist = TokHist{d_hist, cap, 1}; a.counter = d_counter; a.err = d_err; a.polls = S1_SPINS;
     s1.smem = smem;
     s1.stages = 1;
     for (const LayerW& l : layers) s1.stages += l.attn ? 7 : 6;
@@ -2576,6 +2576,15 @@ int b2_debug_step1_plan(const char* config_json, int sms, int has_keys, int kv_d
                 }
             }
     return n;
+}
+
+int b2_debug_step1_polls(b2_engine* e, int polls) {
+    if (!e || !e->finished) return 1;
+    if (polls < 0 || polls > S1_SPINS) return e->fail("polls outside 0..%d", S1_SPINS);
+    CUE(cudaSetDevice(e->device));
+    CUE(cudaStreamSynchronize(e->stream));
+    e->s1.args.polls = polls ? polls : S1_SPINS;
+    return e->build_graph();
 }
 
 int b2_debug_trace_step(b2_engine* e, unsigned long long* out, int cap_launches, int* n_launches) {

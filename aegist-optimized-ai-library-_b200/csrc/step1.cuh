@@ -103,6 +103,7 @@ struct Step1Args {
     const float *rope_cos, *rope_sin;
     const int* page_table;
     float scale, eps;
+    uint32_t polls;              // before a wait gives up; at least 1
     int L, V, E, topk, I, SH, HK, HV, DV, H, KV, RD, C, n1, n2, cores_k, kv_f32, kv_tile, head_rows, half_i8, half_bf, half_out, half_pair, half_shd, nst, stage_bytes;
     size_t expert_bytes, off_gu_s, off_gu_m, off_dn_q, off_dn_s, off_dn_m;
     float *cscore, *cselw;
@@ -134,12 +135,12 @@ __device__ __forceinline__ void ll_again2(const uint64_t* p, uint32_t tag, uint6
     asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, %4;\n setp.ne.or.u32 q, %3, %4, q;\n @q ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%5];\n}"
                  : "+l"(r0), "+l"(r1) : "r"((uint32_t)(r0 >> 32)), "r"((uint32_t)(r1 >> 32)), "r"(tag), "l"(p) : "memory");
 }
-// Waits are bounded: one that has polled S1_SPINS times raises the block's flag, all later waits of the block give up at once, and at the
+// Waits are bounded: one that has polled Step1Args::polls times raises the block's flag, all later waits of the block give up at once, and at the
 // end the block reports it. (Blocks that wait for this one then get words that mean nothing, and come to their end.)
 __device__ __forceinline__ bool s1_given_up(int spin, uint32_t flag) {
-    uint32_t f;
-    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(f) : "r"(flag) : "memory");
-    if (spin == S1_SPINS) { f = 1u; asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(flag), "r"(f) : "memory"); }
+    uint32_t f, polls;
+    asm volatile("ld.volatile.shared.v2.u32 {%0, %1}, [%2];" : "=r"(f), "=r"(polls) : "r"(flag) : "memory");
+    if ((uint32_t)spin >= polls) { f = 1u; asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(flag), "r"(f) : "memory"); }
     return __any_sync(0xffffffffu, f != 0u);
 }
 // N neighbouring values per lane, and M more at q, by a whole warp; lanes without need go along. N, M = 1 or even (then 16-byte aligned)
@@ -792,12 +793,13 @@ __global__ void __launch_bounds__(S1_THREADS, 1) k_step1(const __grid_constant__
     __shared__ int s_top[8], s_page[S1_PAGES], s_last;
     __shared__ S1Block s_blk;
     __shared__ float s_rope[HD];                       // cosines | sines of this position
-    __shared__ uint32_t s_given_up;                    // a wait of this block has run out
+    __shared__ __align__(8) uint32_t s_given_up[2];    // a wait of this block has run out | after so many polls
     int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, tid = lane & 3;
     const int blk = blockIdx.x, G = gridDim.x;
 
     if (threadIdx.x == 0) {
-        s_given_up = 0u;
+        s_given_up[0] = 0u;
+        s_given_up[1] = a.polls;
         mbar_init(&s_picked, 1);
         for (int s = 0; s < a.nst; s++) { mbar_init(&s_bars[s], 1); mbar_init(&s_bars[S1_MAXST + s], S1_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -842,7 +844,7 @@ __global__ void __launch_bounds__(S1_THREADS, 1) k_step1(const __grid_constant__
     }
     __syncthreads();
 
-    const uint32_t bars = held(smem_u32(s_bars)), ring0 = smem_u32(ring), flag = held(smem_u32(&s_given_up));
+    const uint32_t bars = held(smem_u32(s_bars)), ring0 = smem_u32(ring), flag = held(smem_u32(s_given_up));
     if (warp >= S1_WARPS) {
         regs_dec<S1_REGS_LOW>();
         if (warp > S1_WARPS) {
@@ -1692,7 +1694,7 @@ __global__ void __launch_bounds__(S1_THREADS, 1) k_step1(const __grid_constant__
         if (lane == 0) {
             a.part_val[blk] = v;
             a.part_idx[blk] = ix;
-            if (s_given_up) atomicExch(a.err, 4);
+            if (s_given_up[0]) atomicExch(a.err, 4);
             __threadfence();
             s_last = atomicAdd(a.counter, 1u) == (unsigned)G - 1;
             __threadfence();

@@ -86,6 +86,7 @@ SYMBOLS = {
     "b2_stages_per_step": (_I, [_P]),
     "b2_debug_umma_launches": (C.c_long, []),
     "b2_debug_refuse_tensor_maps": (None, [_I]),
+    "b2_debug_step1_polls": (_I, [_P, _I]),
     "b2_debug_step1_plan": (_I, [C.c_char_p, _I, _I, _I, C.POINTER(C.c_int64), _I]),
     "b2_step_bytes": (C.c_double, [_P]),
     "b2_ep_bytes_per_step": (C.c_double, [_P]),
@@ -409,6 +410,10 @@ class HybridEngine:
     def stages_per_step(self) -> int:
         """Rows of a step's timeline: its launches, or the stages inside the one launch."""
         return self._lib.b2_stages_per_step(self._h)
+
+    def set_step1_polls(self, polls: int = 0):
+        """Polls before a wait inside the persistent step gives up (see b2_debug_step1_polls); 0: the default."""
+        self._check(self._lib.b2_debug_step1_polls(self._h, polls))
 
     def step_bytes(self) -> float:
         return self._lib.b2_step_bytes(self._h)

@@ -171,6 +171,9 @@ long b2_debug_umma_launches(void);
  * the number of records (`out` holds 9 * cap words), 0 where the step runs as launches, -1 for a config that no engine takes.
  * No counterpart in the reference. */
 int b2_debug_step1_plan(const char* config_json, int sms, int has_keys, int kv_dtype, int64_t* out, int cap);
+/* Polls before a wait inside the persistent step gives up, which ends the step with an error and leaves a state that is good for
+ * nothing but b2_crop(0); 0 is the default, about a second. For tests of that. No counterpart in the reference. */
+int b2_debug_step1_polls(b2_engine* e, int polls);
 /* While on, the calling thread's engines and operators are refused every tensor map, as a driver could: the kernels
  * that need none run instead. For tests of that fall-back. No counterpart in the reference. */
 void b2_debug_refuse_tensor_maps(int on);

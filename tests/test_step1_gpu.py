@@ -140,10 +140,12 @@ def test_brain_without_core_engine(E, pkg, monkeypatch, which):
 @gpu
 @pytest.mark.parametrize("kv", ["f32", "bf16"])
 @pytest.mark.parametrize("name,context", [("half", 1), ("half", 15), ("half", 1184), ("narrow", 17), ("full", 16), ("full", 63),
-                                          ("full", 64), ("full", 1183), ("full", 1185), ("full", 4800)])
+                                          ("full", 64), ("full", 1183), ("full", 1185), ("full", 4800),
+                                          ("full", 4142), ("full", 8434), ("full", 16900), ("half", 8300)])
 def test_attention_slices(E, pkg, monkeypatch, name, context, kv):
-    """Slices of 16 positions up to 16 x 74 (blocks per KV head), longer ones behind; page borders; a block's second pass over its slice
-    (more than two tiles of keys)."""
+    """Slices of 16 positions up to 16 x 74 (blocks per KV head), longer ones behind; page borders. A block's pass over its slice is two tiles
+    of keys: at full width 56 positions of an fp32 cache, 114 of bf16. 4142 and 8434 cross 74 times that within three tokens; 8434 (fp32)
+    and 16900 have a third pass."""
     cfg = shape(pkg, name, 4)
     one, many = pair(E, pkg, monkeypatch, cfg, E.KV_F32 if kv == "f32" else E.KV_BF16, context + 16)
     ids = np.random.default_rng(context).integers(0, cfg.vocab_size, context)
@@ -177,6 +179,32 @@ def test_timeline(E, pkg):
     delta, attn = [1, 3, 1, 1, 5, 6], [1, 7, 8, 1, 1, 5, 6]          # in-projections, mixer (and merge), out, router, gate/up, down
     assert t[:, 5].tolist() == 3 * delta + attn + [1]
     assert (t[:, 4] > t[:, 0]).all() and (np.diff(t[:, 4]) > 0).all()      # a stage ends after it began, and after the one before
+    e.close()
+
+
+@gpu
+@pytest.mark.parametrize("polls", [1, 2, 40])
+def test_waits_that_run_out(E, pkg, polls):
+    """Fewer polls than a value takes to come: the step ends with an error, no wait lasts, and the engine works again after it."""
+    from b200moe import brain
+    cfg = shape(pkg, "half", 4)
+    e = E.HybridEngine.from_tensors(cfg.to_dict(), brain.random_brain(cfg, seed=1, device="cuda:0"), max_context=1300, device=0, batch=1, kv_dtype=E.KV_F32)
+    ids = np.arange(1200) % cfg.vocab_size
+    e.feed(ids, want_logits=False)
+    want = np.array(e.feed([7]))
+    e.set_step1_polls(polls)
+    errors = 0
+    for _ in range(3):
+        try:
+            e.feed([8])
+        except E.EngineError as x:
+            assert "waited too long" in str(x)
+            errors += 1
+    assert errors == 3 or polls > 2
+    e.set_step1_polls()
+    assert e.crop(0) == 0
+    e.feed(ids, want_logits=False)
+    assert np.array_equal(np.array(e.feed([7])), want)
     e.close()
 
 
