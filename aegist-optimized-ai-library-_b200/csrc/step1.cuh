@@ -16,12 +16,14 @@
 // Every sum is added in the order and with the roundings of the kernels that run steps of two to five sequences, so that a sequence has
 // the same bits beside others as alone: slices, chunks and groups below are cut as there. (A sixteenth of the contraction per warp, with
 // the rms behind the products and a scale for every slice, is 1.1x faster.) Only the attention's split of the context differs.
-// The launch is cooperative: its blocks wait on one another, so all of them must be resident. Every wait is bounded; one that
-// runs out sets the error word and lets the step run to its end.
+// The launch is cooperative: its blocks wait on one another, so all of them must be resident, and it begins when they can be (behind a
+// kernel that held one SM for 2.5 s it took 2.5 s and no wait ran out). Every wait is bounded; one that runs out sets the error
+// word and lets the step run to its end.
 //
 // Buffers that carry tagged words are used again two layers later. A block that writes for layer l + 2 has read all rows of
 // layer l + 1's output, and every block owns some of those (rows are spread over all blocks), written after that block's last
-// read of layer l.
+// read of layer l. The attention's partial results have one place for all layers: who writes them for layer l + 1 has read all of layer
+// l's output, which every block wrote after its last read of that layer's.
 #pragma once
 
 namespace b2 {

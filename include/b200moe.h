@@ -6,7 +6,9 @@
  * ids are u32, logits are f32[vocab], errors are a non-zero return code plus a message
  * (`b2_last_error`), never an abort.
  *
- * Threading: one engine is used by one thread at a time (the reference takes `&mut self`).
+ * Threading: one engine is used by one thread at a time (the reference takes `&mut self`); engines of several
+ * threads are independent. While one of them is opened or captures a step (b2_finish, b2_open, b2_set_taps, b2_debug_*), no
+ * thread of the process may wait for the whole device (cudaDeviceSynchronize): CUDA breaks such captures off.
  * All functions returning int return 0 on success.
  */
 #ifndef B200MOE_H
