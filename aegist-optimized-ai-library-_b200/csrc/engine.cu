@@ -20,7 +20,6 @@
 #include <map>
 #include <memory>
 #include <mutex>
-#include <set>
 #include <string>
 #include <vector>
 
@@ -697,22 +696,24 @@ static cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
     return launch_kc(1, kernel, grid, block, smem, st, args...);
 }
 
-// The limit belongs to the kernel on its device, and engines of several threads ask for different sizes: always all there is, once.
+// The limit belongs to the kernel on its device, and engines of several threads ask for different sizes: always all there is. (Set every time: a
+// host program may have reset the device between two engines.)
 template <typename F>
 static cudaError_t opt_in_smem(F* f, size_t bytes) {
     if (bytes <= 32 * 1024) return cudaSuccess;        // the 48 KB that need no opting in hold the kernel's static arrays too
     static std::mutex mutex;
-    static std::set<std::pair<int, const void*>> known;
-    int device;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lock(mutex);
-    if (known.count({device, (const void*)f})) return cudaSuccess;
-    cudaFuncAttributes fa;
-    e = cudaFuncGetAttributes(&fa, (const void*)f);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes);
-    if (e == cudaSuccess) known.insert({device, (const void*)f});
-    return e;
+    static std::map<const void*, int> limits;
+    std::unique_lock<std::mutex> lock(mutex);
+    int& limit = limits[(const void*)f];
+    if (!limit) {
+        cudaFuncAttributes fa;
+        const cudaError_t e = cudaFuncGetAttributes(&fa, (const void*)f);
+        if (e != cudaSuccess) return e;
+        limit = 227 * 1024 - (int)fa.sharedSizeBytes;
+    }
+    const int all = limit;
+    lock.unlock();
+    return cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, all);
 }
 
 // k_mma_i8 over `passes` groups of MM_TOK sequences. A grid that gives an SM at most one block (the out projections,
