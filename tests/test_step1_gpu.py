@@ -140,12 +140,10 @@ def test_brain_without_core_engine(E, pkg, monkeypatch, which):
 @gpu
 @pytest.mark.parametrize("kv", ["f32", "bf16"])
 @pytest.mark.parametrize("name,context", [("half", 1), ("half", 15), ("half", 1184), ("narrow", 17), ("full", 16), ("full", 63),
-                                          ("full", 64), ("full", 1183), ("full", 1185), ("full", 4800),
-                                          ("full", 4142), ("full", 8434), ("full", 16900), ("half", 8300)])
+                                          ("full", 64), ("full", 1183), ("full", 1185), ("full", 4800)])
 def test_attention_slices(E, pkg, monkeypatch, name, context, kv):
-    """Slices of 16 positions up to 16 x 74 (blocks per KV head), longer ones behind; page borders. A block's pass over its slice is two tiles
-    of keys: at full width 56 positions of an fp32 cache, 114 of bf16. 4142 and 8434 cross 74 times that within three tokens; 8434 (fp32)
-    and 16900 have a third pass."""
+    """Slices of 16 positions up to 16 x 74 (blocks per KV head), longer ones behind; page borders; a block's second pass over its slice
+    (more than two tiles of keys)."""
     cfg = shape(pkg, name, 4)
     one, many = pair(E, pkg, monkeypatch, cfg, E.KV_F32 if kv == "f32" else E.KV_BF16, context + 16)
     ids = np.random.default_rng(context).integers(0, cfg.vocab_size, context)
@@ -156,6 +154,15 @@ def test_attention_slices(E, pkg, monkeypatch, name, context, kv):
         a, b = (np.array(e.feed([tok])) for e in (one, many))
         assert np.isfinite(a).all() and np.abs(a - b).max() < tol
     one.close(); many.close()
+
+
+@gpu
+@pytest.mark.parametrize("kv", ["f32", "bf16"])
+@pytest.mark.parametrize("name,context", [("full", 4142), ("full", 8434), ("full", 16900), ("half", 8300)])
+def test_attention_passes(E, pkg, monkeypatch, name, context, kv):
+    """A block's pass over its slice is two tiles of keys: at full width 56 positions of an fp32 cache, 114 of bf16. 4142 and 8434 cross
+    74 times that within three tokens; 8434 (fp32) and 16900 have a third pass."""
+    test_attention_slices(E, pkg, monkeypatch, name, context, kv)
 
 
 @gpu
