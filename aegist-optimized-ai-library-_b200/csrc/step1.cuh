@@ -1459,9 +1459,6 @@ __global__ void __launch_bounds__(S1_THREADS, 1) k_step1(const __grid_constant__
             const int gp0 = s_blk.gp0, np = s_blk.gp1 - gp0;
             tr.in(5, np);
             if (warp == 0) {
-                // softmax over E <= 256 logits, the topk <= 8 largest in descending order, ties to the lower index (aegist/hybrid.py:641-645): a
-                // probability is positive, so its bits order like an integer. A lane holds eight neighbouring experts, sorted; a round is
-                // one reduction over the lanes' first ones
                 float lg[8];
                 const bool has = lane * 8 < a.E;
                 ll_wait<8>(set + a.o_rl + lane * 8, tag, has, lg, flag);
